@@ -863,12 +863,13 @@ bool enqueue_query_split(const Engine *e, const Batch *bt, const uint8_t *d_slot
 bool enqueue_scan_tails(Engine *e, Batch *bt, const Plan &p, const CUtensorMap &map_q, const uint8_t *d_slots,
                         size_t slot_stride, size_t slots, uint8_t *resp, size_t resp_stride, const Groups &gr,
                         const cudaEvent_t *done, int *launches, cudaEvent_t before_last_tail = nullptr,
-                        cudaEvent_t last_tail_after = nullptr, int inline_from = 8, int kb_lo = 0) {
-  cudaStream_t st = bt->st;
+                        cudaEvent_t last_tail_after = nullptr, int inline_from = 8, int kb_lo = 0,
+                        bool scan_on_side = false) {
+  cudaStream_t st = bt->st, ss = scan_on_side ? bt->side : st;
   bool forked = false;
   for (int g = 0; g < gr.count; ++g) {
     const int o0 = gr.bounds[g], parts = gr.bounds[g + 1] - o0;
-    const bool ok = gr.count == 1 ? launch_scan(e, p, map_q, bt->d_acc, slots, st, bt->d_err, 0, -1, kb_lo)
+    const bool ok = gr.count == 1 ? launch_scan(e, p, map_q, bt->d_acc, slots, ss, bt->d_err, 0, -1, kb_lo)
                                   : launch_scan(e, p, map_q, bt->d_acc, slots, st, bt->d_err, o0 * gr.tiles_per_part,
                                                 parts * gr.tiles_per_part, kb_lo);
     if (!ok) return false;
@@ -878,8 +879,12 @@ bool enqueue_scan_tails(Engine *e, Batch *bt, const Plan &p, const CUtensorMap &
       ALTO_CK(cudaEventRecord(bt->ev_scan[g], st));
       ALTO_CK(cudaStreamWaitEvent(ts, bt->ev_scan[g], 0));
       forked = true;
-    } else if (last && before_last_tail) {
-      ALTO_CK(cudaEventRecord(before_last_tail, st));
+    } else {
+      if (ss != st) {
+        ALTO_CK(cudaEventRecord(bt->ev_scan[g], ss));
+        ALTO_CK(cudaStreamWaitEvent(st, bt->ev_scan[g], 0));
+      }
+      if (last && before_last_tail) ALTO_CK(cudaEventRecord(before_last_tail, st));
     }
     if (last_tail_after && ts == st) ALTO_CK(cudaStreamWaitEvent(st, last_tail_after, 0));
     ALTO_CK(alto::launch_tail(tail_args(e, bt, d_slots, slot_stride, resp, resp_stride, o0, parts), slots, ts));
@@ -903,12 +908,19 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
                           uint8_t *resp, size_t resp_stride, bool host_status, bool with_marks) {
   cudaStream_t st = bt->st;
   const Plan p = make_plan(e, slots);
-  const Groups groups = column_groups(e, p, group_weights(e->overlap ? e->groups : 1, false));
+  // A batch of few response bytes scans in one launch, as in answer_host.  With the single-CTA kernels (HBM-bound, two
+  // CTAs an SM) the scan also follows its query split on the side stream without waiting for the pack: its units fill
+  // the SMs as the pack's run out, instead of starting on an idle device after the pack's last one.  One frame over
+  // 1 GiB: 376 -> 336 us a call (6.4 TB/s of database and packing matrix); alto_answer 404 -> 358, 251 -> 221 at 64 MiB.
+  const bool grouped = e->overlap && slots * e->resp_len >= kGroupedRespBytes;
+  const Groups groups = column_groups(e, p, group_weights(grouped ? e->groups : 1, false));
+  const bool scan_on_side = e->overlap && !p.pair && groups.count == 1;
   const int bp = (int)round_up(slots, 4);
   int launches = 0;
   // timing marks (main batch only): 0 begin | validate (one stream only) | 1 | y split | 2 | pack | 3 | (wait for
   // the side stream) | 4 | scan (with all tails but the last beside it) | 5 | last tail | 6.  With two streams the
-  // intervals are the exposed times: validation and the query split run beside the key split and the pack.
+  // intervals are the exposed times: validation and the query split run beside the key split and the pack, and a small
+  // batch's scan (scan_on_side) counts from the end of the pack.
   cudaEvent_t *mk = nullptr;
   if (bt->timing && with_marks) {
     int set = 0;
@@ -950,7 +962,9 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
   if (!launch_pack(e, p, map_y, bt->d_beta, slots, st, bt->d_err)) return false;
   ++launches;
   ALTO_CK(mark(3));
-  if (e->overlap) {
+  if (scan_on_side) {
+    // the scan follows the query split on the side stream
+  } else if (e->overlap) {
     ALTO_CK(cudaStreamWaitEvent(st, bt->ev_qready, 0));
   } else {
     if (!enqueue_query_split(e, bt, d_slots, slot_stride, slots, st)) return false;
@@ -958,8 +972,7 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
   }
   ALTO_CK(mark(4));
   if (!enqueue_scan_tails(e, bt, p, map_q, d_slots, slot_stride, slots, resp, resp_stride, groups, nullptr,
-                          &launches,
-                          mk ? mk[5] : nullptr))
+                          &launches, mk ? mk[5] : nullptr, nullptr, 8, 0, scan_on_side))
     return false;
   ALTO_CK(mark(6));
   e->last_launches = launches;
@@ -1198,6 +1211,10 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
   // status download once the z keys are: on the side stream beside the pack (on the batch's stream after the pack
   // without the overlap).  The scans wait for the split only; the last tail also waits for the statuses.
   cudaStream_t vs = e->overlap ? bt->side : st;
+  // A small batch's scan follows its query split on the side stream, so validation waits for the z keys on the copy
+  // stream instead.
+  const bool scan_on_side = e->overlap && !p.pair && !piped && groups.count == 1;
+  cudaStream_t zs = scan_on_side ? sc : vs;
   if (!piped) {
     ALTO_H(cudaStreamWaitEvent(vs, e->ev_queries, 0));
     if (!enqueue_query_split(e, bt, bt->d_req, e->slot_stride, nc, vs)) return -4;
@@ -1218,13 +1235,13 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
       ALTO_H(cudaEventRecord(e->ev_sgrp[k], vs));
     }
   }
-  ALTO_H(cudaStreamWaitEvent(vs, e->ev_zkeys, 0));
-  alto::validate_kernel<<<(unsigned)nc, 256, 0, vs>>>(bt->d_req, e->slot_stride, kSlotLead, e->count, e->rows,
+  ALTO_H(cudaStreamWaitEvent(zs, e->ev_zkeys, 0));
+  alto::validate_kernel<<<(unsigned)nc, 256, 0, zs>>>(bt->d_req, e->slot_stride, kSlotLead, e->count, e->rows,
                                                       bt->d_status);
   ALTO_H(cudaGetLastError());
   ++launches;
-  ALTO_H(cudaMemcpyAsync(bt->h_status, bt->d_status, nc * sizeof(int), cudaMemcpyDeviceToHost, vs));
-  ALTO_H(cudaEventRecord(e->ev_status, vs));
+  ALTO_H(cudaMemcpyAsync(bt->h_status, bt->d_status, nc * sizeof(int), cudaMemcpyDeviceToHost, zs));
+  ALTO_H(cudaEventRecord(e->ev_status, zs));
   // The scan in column groups (with the tails and downloads) covers the last quarter of the chunk groups, which it
   // starts once all query words are in; the chunk groups before it scan all columns as they arrive.  The upload of
   // the query words takes about three quarters of the scan's time (link bytes against int8 work per query word at
@@ -1245,11 +1262,12 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
     group_rows(qtail, &r0, &r1);
     ALTO_H(cudaStreamWaitEvent(st, e->ev_sgrp[qgroups - 1], 0));
     kb_last = (int)(r0 / alto::kBK);
-  } else if (e->overlap) {
+  } else if (e->overlap && !scan_on_side) {
     ALTO_H(cudaStreamWaitEvent(st, bt->ev_qready, 0));
   }
   if (!enqueue_scan_tails(e, bt, p, map_q, bt->d_req, e->slot_stride, nc, bt->d_resp, e->resp_len, groups,
-                          e->ev_group, &launches, nullptr, e->ev_status, groups.count - e->host_inline - 1, kb_last))
+                          e->ev_group, &launches, nullptr, e->ev_status, groups.count - e->host_inline - 1, kb_last,
+                          scan_on_side))
     return -4;
   // the error word comes back behind the last tail, so the final synchronisation covers it
   ALTO_H(cudaMemcpyAsync(bt->h_err, bt->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

@@ -56,7 +56,13 @@ struct GemmShape {
   static constexpr int kABytes = kBM * kBK;
   static constexpr int kBBytes = BN * kBK;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = (196608 / kStageBytes) < 8 ? (196608 / kStageBytes) : 8;
+  // BN = 16 (batches of up to 4 frames) is bound by HBM: two CTAs share an SM, six stages each, so that one CTA's set-up
+  // (barriers, TMEM, first loads) and epilogue hide behind the other's streaming; with one CTA of eight stages the 1 GiB
+  // packing matrix streamed at 6.5 TB/s in 1024 units and half the database at 6.0 TB/s in 384 (three CTAs of four
+  // stages measure the same as two).
+  static constexpr int kCtasPerSm = BN == 16 ? 2 : 1;
+  static constexpr int kRing = kCtasPerSm == 2 ? 110592 : 196608;
+  static constexpr int kStages = (kRing / kStageBytes) < 8 ? (kRing / kStageBytes) : 8;
   static constexpr int kTmemCols = BN < 32 ? 32 : BN;
   static constexpr int kBarrierBytes = 256;
   static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;  // +1024 for manual alignment
@@ -66,7 +72,7 @@ struct GemmShape {
 };
 
 template <int BN, Epi EPI>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kGemmThreads, GemmShape<BN>::kCtasPerSm)
     limb_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      GemmArgs args) {
   using S = GemmShape<BN>;
