@@ -2000,9 +2000,9 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   // n = 2048 with one digit a CTA: the walk with register transforms (ALTO_OFFLINE_WALK8=0 runs the other)
   bool walk8 = n == 2048 && cluster == (int)tg;
   if (const char *v = getenv("ALTO_OFFLINE_WALK8")) walk8 = walk8 && v[0] != '0';
-  const size_t walk8_smem = (2 + 2 * (size_t)cluster) * n * sizeof(uint32_t);
+  const size_t walk8_smem = (3 + 2 * (size_t)cluster) * n * sizeof(uint32_t);
   if (walk8)
-    step(cudaFuncSetAttribute(alto::offline_walk8_kernel<11>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    step(cudaFuncSetAttribute(alto::offline_walk8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)walk8_smem));
   const unsigned nt = (unsigned)std::max<size_t>(32, std::min<size_t>(256, n / 2));
   // walk and finish threads: at least n / 4 (the cluster walk gathers 4 slots a thread ahead), at most 1024
@@ -2048,11 +2048,11 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       if (walk8) {  // n = 2048, one digit a CTA: both transforms in registers
-        cfg.blockDim = dim3((unsigned)(n / 8));
+        cfg.blockDim = dim3((unsigned)(n / 4));
         cfg.dynamicSmemBytes = walk8_smem;
-        step(cudaLaunchKernelEx(&cfg, alto::offline_walk8_kernel<11>, (const uint32_t *)d_act, (int)tg, bits,
+        step(cudaLaunchKernelEx(&cfg, alto::offline_walk8_kernel, (const uint32_t *)d_act, bits,
                                 (const uint32_t *)d_w, (const uint32_t *)d_psi, (const uint32_t *)d_psi_inv, n_inv,
-                                d_bt, d_last));
+                                d_bt, d_last, e->main.d_err));
       } else {
         step(cudaLaunchKernelEx(&cfg, alto::offline_walk_cluster_kernel, (const uint32_t *)d_act, (int)n, logn,
                                 (int)tg, bits, (const uint32_t *)d_w, (const uint32_t *)d_psi,
@@ -2072,6 +2072,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
     step(cudaGetLastError());
     // the engine's tail twiddles: its inverse table psi^-brv / 2, doubled as create_engine stores it
     step(cudaMemcpyAsync(e->d_tw, d_psi_inv, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, 0));
+    step(cudaMemcpyAsync(e->main.h_err, e->main.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, 0));
     step(cudaEventRecord(t1, 0));
     step(cudaEventSynchronize(t1));
   }
@@ -2099,7 +2100,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
     set_error("alto_engine_offline", err);
     return -4;
   }
-  return 0;
+  return check_batch_error(&e->main) ? 0 : -4;  // a wait of the walk between its CTAs ran out
 }
 
 int alto_engine_fill_synthetic(void *p) {

@@ -48,6 +48,38 @@ ALTO_HD uint64_t fold_q64(uint64_t x) { return (x >> 32) * kFold + (x & 0xffffff
 // (a * b) mod Q for any 32-bit a, b.
 ALTO_HD uint32_t mul_q(uint32_t a, uint32_t b) { return red_q64((uint64_t)a * b); }
 
+// Montgomery products: mont_q(a, w 2^32 mod Q) = a w mod Q in [0, Q), for any 32-bit a and w in [0, Q).  With m = lo(x)
+// Q^-1 mod 2^32 the low words of x = a w and m Q agree, so (x - m Q) / 2^32 = hi(x) - hi(m Q), above -Q and below Q
+// (hi(x) < Q as a < 2^32).  Three multiplications and a conditional add, against four multiplications with their 64-bit
+// additions for mul_q, whose operands need no preparation.
+constexpr uint32_t inv_mod_2_32(uint32_t a) {  // a^-1 mod 2^32 for odd a: Newton's iteration from a a = 1 (mod 8)
+  uint32_t x = a;
+  for (int i = 0; i < 4; ++i) x *= 2u - a * x;
+  return x;
+}
+constexpr uint32_t kQInv = inv_mod_2_32(kQ32);
+static_assert(kQInv * kQ32 == 1u, "Q^-1 mod 2^32");
+ALTO_HD uint32_t mont_q(uint32_t a, uint32_t wm) {
+  const uint64_t x = (uint64_t)a * wm;
+  const uint32_t hi = (uint32_t)(x >> 32), h = (uint32_t)(((uint64_t)((uint32_t)x * kQInv) * kQ32) >> 32);
+  const uint32_t r = hi - h;
+  return hi < h ? r + kQ32 : r;
+}
+ALTO_HD uint32_t to_mont(uint32_t w) { return mul_q(w, kFold); }  // w 2^32 mod Q
+
+// Sums and differences that stay below 2^32 without reaching [0, Q): a any 32-bit representative, b in [0, Q).
+// a + b < 2^33 - 12287, so on a carry the low word plus 12287 does not wrap; a - b > -Q, so on a borrow the low word is
+// above 12287.  canon_q brings any 32-bit representative into [0, Q).
+ALTO_HD uint32_t lazy_add(uint32_t a, uint32_t b) {
+  const uint32_t s = a + b;
+  return s < a ? s + kFold : s;
+}
+ALTO_HD uint32_t lazy_sub(uint32_t a, uint32_t b) {
+  const uint32_t d = a - b;
+  return a < b ? d - kFold : d;
+}
+ALTO_HD uint32_t canon_q(uint32_t a) { return umin_u32(a, a - kQ32); }
+
 // 2^-l mod Q: (Q + 1) / 2 is the inverse of 2.
 ALTO_HD uint32_t inv_pow2_q(int l) {
   uint32_t r = 1;

@@ -28,6 +28,7 @@
 #include "hint.cuh"
 #include "kernels.cuh"
 #include "modq.cuh"
+#include "sm100.cuh"
 
 namespace alto {
 
@@ -334,121 +335,226 @@ __global__ void __launch_bounds__(1024) offline_walk_cluster_kernel(const uint32
     for (int s = threadIdx.x; s < n; s += blockDim.x) last[(size_t)chain * n + s] = cur[s];
 }
 
-// The cluster walk with both transforms in registers, for tg CTAs a cluster (one digit each) and n = 2^L: n / 8
-// threads hold 8 values each.  The inverse transform runs the tail kernel's Gentleman-Sande rounds (tail_round: the
-// thread's 8 consecutive slots first, then three stages per shared-memory exchange); the digit goes back through
-// shared memory in natural order and the forward transform runs fwd_round's Cooley-Tukey rounds; the thread then holds
-// slots 8 g .. 8 g + 7 of the next r_i in registers.  Every exchange is double-buffered (one barrier each).
-template <int L>
-__global__ void __launch_bounds__((1 << L) / 8) offline_walk8_kernel(const uint32_t *__restrict__ ev, int tg,
-                                                                     int bits, const uint32_t *__restrict__ w,
-                                                                     const uint32_t *__restrict__ psi,
-                                                                     const uint32_t *__restrict__ psi_inv,
-                                                                     uint32_t n_inv, uint32_t *__restrict__ bt,
-                                                                     uint32_t *__restrict__ last) {
+// ------------------------------------------------------------------------------------ register transforms, n = 2048
+// 512 threads hold 4 values each.  Layout s: index i = (g >> s) << (s + 2) | m << s | (g & (2^s - 1)), so a thread's four
+// values differ in bits s and s + 1.  The inverse transform runs two stages in each of the layouts 0, 2, 4, 6, 8 and the
+// last one (t = 1024) in layout 9; the forward transform the same backwards.  Between layouts the values go through
+// shared memory at swz4(i), free of bank conflicts in every layout.  0 <-> 2 <-> 4 stay inside a warp, 4 <-> 6 inside
+// two warps and 6 <-> 8 inside eight, so that only 8 <-> 9 needs a barrier of the whole block.  Twiddles are in
+// Montgomery form.
+struct RegTwiddles {
+  uint32_t c[5], a[5][2], d;  // per layout: the stage of bit s + 1, the two of bit s; the last stage
+};
+__device__ __forceinline__ void load_tw(RegTwiddles &t, const uint32_t *__restrict__ psi, int g) {
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int base = (2048 >> (2 * q + 2)) + (g >> (2 * q));
+    t.c[q] = to_mont(__ldg(psi + base));
+    t.a[q][0] = to_mont(__ldg(psi + 2 * base));
+    t.a[q][1] = to_mont(__ldg(psi + 2 * base + 1));
+  }
+  t.d = to_mont(__ldg(psi + 1));
+}
+
+// Two butterflies each: Gentleman-Sande on residues, Cooley-Tukey on 32-bit representatives (lazy_add).
+__device__ __forceinline__ void bf_gs(uint32_t &x, uint32_t &y, uint32_t wm) {
+  const uint32_t s = add_q(x, y);
+  y = mont_q(sub_q(x, y), wm);
+  x = s;
+}
+__device__ __forceinline__ void bf_ct(uint32_t &x, uint32_t &y, uint32_t wm) {
+  const uint32_t v = mont_q(y, wm);
+  y = lazy_sub(x, v);
+  x = lazy_add(x, v);
+}
+
+__device__ __forceinline__ int swz4(int i) { return i ^ (((i >> 5) & 1) << 2) ^ (((i >> 6) & 1) * 0x18); }
+template <int S>
+__device__ __forceinline__ int reg_index(int g, int m) {
+  return ((g >> S) << (S + 2)) | (m << S) | (g & ((1 << S) - 1));
+}
+template <int S>
+__device__ __forceinline__ void put4(uint32_t *buf, const uint32_t (&x)[4], int g) {
+  if constexpr (S == 0) {
+    *reinterpret_cast<uint4 *>(buf + swz4(4 * g)) = make_uint4(x[0], x[1], x[2], x[3]);
+  } else {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) buf[swz4(reg_index<S>(g, m))] = x[m];
+  }
+}
+template <int S>
+__device__ __forceinline__ void get4(const uint32_t *buf, uint32_t (&x)[4], int g) {
+  if constexpr (S == 0) {
+    const uint4 u = *reinterpret_cast<const uint4 *>(buf + swz4(4 * g));
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+  } else {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) x[m] = buf[swz4(reg_index<S>(g, m))];
+  }
+}
+__device__ __forceinline__ void sync_warps(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// Moves the values from layout A to layout B through `buf`, behind a barrier of the threads that share words.
+template <int A, int B>
+__device__ __forceinline__ void relayout(uint32_t (&x)[4], uint32_t *buf, int g) {
+  constexpr int S = A < B ? A : B;
+  put4<A>(buf, x, g);
+  if constexpr (S < 4) __syncwarp();
+  else if constexpr (S == 4) sync_warps(1 + (g >> 6), 64);
+  else if constexpr (S == 6) sync_warps(9 + (g >> 8), 256);
+  else __syncthreads();
+  get4<B>(buf, x, g);
+}
+__device__ __forceinline__ void round_gs(uint32_t (&x)[4], const RegTwiddles &t, int q) {
+  bf_gs(x[0], x[1], t.a[q][0]);
+  bf_gs(x[2], x[3], t.a[q][1]);
+  bf_gs(x[0], x[2], t.c[q]);
+  bf_gs(x[1], x[3], t.c[q]);
+}
+__device__ __forceinline__ void round_ct(uint32_t (&x)[4], const RegTwiddles &t, int q) {
+  bf_ct(x[0], x[2], t.c[q]);
+  bf_ct(x[1], x[3], t.c[q]);
+  bf_ct(x[0], x[1], t.a[q][0]);
+  bf_ct(x[2], x[3], t.a[q][1]);
+}
+
+// Residues in layout 0 in, residues in layout 9 out (without n^-1).  Two buffers of 2048 words, used in turn: a buffer is
+// written again only after a barrier that follows its last reads by every thread sharing the words, here and over calls
+// of the two transforms in turn.
+__device__ __forceinline__ void intt_regs(uint32_t (&x)[4], uint32_t *b0, uint32_t *b1, const RegTwiddles &t, int g) {
+  round_gs(x, t, 0);
+  relayout<0, 2>(x, b0, g);
+  round_gs(x, t, 1);
+  relayout<2, 4>(x, b1, g);
+  round_gs(x, t, 2);
+  relayout<4, 6>(x, b0, g);
+  round_gs(x, t, 3);
+  relayout<6, 8>(x, b1, g);
+  round_gs(x, t, 4);
+  relayout<8, 9>(x, b0, g);
+  bf_gs(x[0], x[2], t.d);
+  bf_gs(x[1], x[3], t.d);
+}
+// 32-bit representatives in layout 9 in, the same in layout 0 out.
+__device__ __forceinline__ void ntt_regs(uint32_t (&x)[4], uint32_t *b0, uint32_t *b1, const RegTwiddles &t, int g) {
+  bf_ct(x[0], x[2], t.d);
+  bf_ct(x[1], x[3], t.d);
+  relayout<9, 8>(x, b1, g);
+  round_ct(x, t, 4);
+  relayout<8, 6>(x, b0, g);
+  round_ct(x, t, 3);
+  relayout<6, 4>(x, b1, g);
+  round_ct(x, t, 2);
+  relayout<4, 2>(x, b0, g);
+  round_ct(x, t, 1);
+  relayout<2, 0>(x, b1, g);
+  round_ct(x, t, 0);
+}
+
+// The cluster walk for n = 2048, tg CTAs a cluster (one digit each), both transforms in registers.  A chain is 1022
+// dependent steps, so a step's time is its instructions and barriers in a row: the twiddles stay in registers for the
+// whole walk, the coefficients leave the inverse transform in the layout that the forward one starts from, and n^-1 is
+// folded into w and the aggregates (x holds n^-1 times the reference's r_i, so the inverse transform gives its
+// coefficients themselves).  Every CTA runs the inverse transform, transforms its own digit, and copies its share of the
+// next r_i -- its digit's product with the rotated w, plus the aggregate of the slots that are its own modulo C -- into
+// every other CTA's shared memory (a 512-byte bulk copy a warp, counted on the receiver's barrier).  The share buffers
+// and their barriers alternate by step: a warp sends its share of step i + 2 after every share of step i + 1 has arrived,
+// which the others' same warps sent after they had received and read step i's.
+// Measured for one walk of 1022 steps (the set-up of 2,048 records x 2,048 bytes): 15.6 ms with twiddles loaded from
+// global memory by 256 threads of 8 values and shares pushed by remote stores before a cluster barrier, 6.7 with the
+// twiddles in registers, Montgomery products and no exchange between the transforms, 6.2 with bulk copies for the
+// remote stores, 4.7 with 512 threads of 4 values (two warps a scheduler left most of the fixed latencies exposed).
+__global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *__restrict__ ev, int bits,
+                                                               const uint32_t *__restrict__ w,
+                                                               const uint32_t *__restrict__ psi,
+                                                               const uint32_t *__restrict__ psi_inv, uint32_t n_inv,
+                                                               uint32_t *__restrict__ bt, uint32_t *__restrict__ last,
+                                                               uint32_t *err) {
   namespace cg = cooperative_groups;
-  constexpr int n = 1 << L, NT = n / 8;
-  constexpr int ls = (L % 3) ? (L % 3) : 3, lt = n >> (L - ls + 1);  // the forward transform's last round
-  extern __shared__ uint32_t osm[];
+  constexpr int n = 2048, half = n / 2;
+  extern __shared__ __align__(16) uint32_t osm[];
+  __shared__ __align__(8) uint64_t arrived[2];
+  __shared__ int bail;
   cg::cluster_group cl = cg::this_cluster();
-  const int C = (int)cl.num_blocks(), k = (int)cl.block_rank();  // this CTA's digit
-  const int chain = blockIdx.x / C, o = chain >> 1, bar = chain & 1, half = n >> 1, g = threadIdx.x;
-  // parts[buffer][rank][slot]: every CTA pushes its share into every CTA's buffer (remote stores do not stall the
-  // thread, where remote loads would), and the buffers alternate by step, so one cluster barrier a step suffices
-  uint32_t *parts = osm + 2 * n;
-  int pb = 0;
-  const uint32_t mask = bits >= 32 ? 0xffffffffu : (1u << bits) - 1u;
+  const int C = (int)cl.num_blocks(), k = (int)cl.block_rank();  // one CTA per gadget digit; this CTA's digit
+  const int chain = blockIdx.x / C, o = chain >> 1, bar = chain & 1, g = threadIdx.x;
+  uint32_t *b0 = osm, *b1 = osm + n, *wk = osm + 2 * n, *parts = osm + 3 * n;  // parts[buffer][rank][slot]
+  const int shift = bits * k < 32 ? bits * k : 0;
+  const uint32_t mask = bits * k < 32 ? (bits >= 32 ? 0xffffffffu : (1u << bits) - 1u) : 0u;
   const uint32_t *evo = ev + (size_t)o * n * n;
-  int ex = 0;
-  uint32_t x[8];
-  int e = gen_pow(half - 1, bar, n);
+  RegTwiddles fw, iv;
+  load_tw(fw, psi, g);
+  load_tw(iv, psi_inv, g);
+  for (int s = g; s < n; s += 512) wk[s] = to_mont(mul_q(__ldg(w + k * n + s), n_inv));
+  const uint32_t agg_scale = to_mont(mul_q(n_inv, n_inv));
+  uint32_t odd[4], own = 0;  // 2 brv(slot) + 1; the thread's slots whose aggregate this CTA adds
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const int sl = 8 * g + m;
-    x[m] = mul_q(evo[(size_t)auto_slot(e, sl, n, L) * n + sl], n_inv);
+  for (int m = 0; m < 4; ++m) {
+    odd[m] = 2u * (__brev((uint32_t)(4 * g + m)) >> 21) + 1u;
+    if ((4 * g + m) % C == k) own |= 1u << m;
   }
+  auto slot_of = [&](uint32_t e, int m) { return __brev(((e * odd[m]) & (2 * n - 1)) >> 1) >> 21; };
+  uint32_t x[4], e = (uint32_t)gen_pow(half - 1, bar, n);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) x[m] = mont_q(evo[(size_t)slot_of(e, m) * n + 4 * g + m], agg_scale);
+  const uint32_t bar0 = smem_u32(arrived);
+  if (g == 0) {
+    mbar_init(bar0, 1);
+    mbar_init(bar0 + 8, 1);
+    bail = 0;
+    fence_barrier_init();
+  }
+  uint32_t *out = bt + (((size_t)chain * (half - 1) + (half - 2)) * C + k) * n + 4 * g;
+  cluster_sync_all();  // w is in shared memory, and every CTA's barriers are ready for the others' shares
+  int pb = 0, phase = 0;
   for (int i = half - 2; i >= 0; --i) {
-    // this step's aggregate r_i (gathered from ev), loaded now so that its latency hides behind the transforms
-    e = gen_pow(i, bar, n);
-    uint32_t agg[8];
+    if (g == 0) mbar_arrive_expect_tx(bar0 + 8 * pb, (uint32_t)((C - 1) * n * 4));
+    // the aggregates are gathered now, so that their latency hides behind the transforms
+    e = (e * 0xcccccccdu) & (2 * n - 1);  // times 5^-1 mod 2n
+    uint32_t agg[4];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int sl = 8 * g + m;
-      agg[m] = evo[(size_t)auto_slot(e, sl, n, L) * n + sl];
+    for (int m = 0; m < 4; ++m)
+      agg[m] = (own >> m) & 1u ? __ldg(evo + (size_t)slot_of(e, m) * n + 4 * g + m) : 0u;
+    intt_regs(x, b0, b1, iv, g);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) x[m] = (x[m] >> shift) & mask;
+    ntt_regs(x, b0, b1, fw, g);
+    uint32_t v[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      x[m] = canon_q(x[m]);
+      v[m] = mont_q(x[m], wk[slot_of(e, m)]);
+      if ((own >> m) & 1u) v[m] = add_q(v[m], mont_q(agg[m], agg_scale));
     }
-    // inverse transform (without n^-1)
-    tail_round<L>(x, g, 0, 3, psi_inv);
-#pragma unroll
-    for (int s0 = 3; s0 < L; s0 += 3) {
-      const int r = (L - s0) < 3 ? (L - s0) : 3;
-      uint32_t *buf = osm + (ex++ & 1) * n;
-#pragma unroll
-      for (int m = 0; m < 8; ++m) buf[tail_swz(tail_index<L>(g, m, s0 - 3, 3))] = x[m];
-      __syncthreads();
-#pragma unroll
-      for (int gi = 0; gi < (8 >> r); ++gi) {
-        uint32_t *y = x + gi * (1 << r);
-#pragma unroll
-        for (int m = 0; m < (1 << r); ++m) y[m] = buf[tail_swz(tail_index<L>(gi * NT + g, m, s0, r))];
-        tail_round<L>(y, gi * NT + g, s0, r, psi_inv);
-      }
+    uint32_t *mine = parts + (size_t)(pb * C + k) * n;
+    reinterpret_cast<uint4 *>(mine)[g] = make_uint4(v[0], v[1], v[2], v[3]);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((g & 31) < C && (g & 31) != k) {  // each warp sends its 128 words as soon as they are written
+      const uint32_t src = smem_u32(mine + 4 * (g & ~31)), r = (uint32_t)(g & 31);
+      bulk_copy_to_cta(map_to_rank(src, r), src, 512, map_to_rank(bar0 + 8 * pb, r));
     }
-    // this CTA's digit, in natural order, to the forward transform's first-round layout
-    {
-      constexpr int s0l = ((L - 1) / 3) * 3, rl = L - s0l;
-      uint32_t *buf = osm + (ex++ & 1) * n;
-#pragma unroll
-      for (int gi = 0; gi < (8 >> rl); ++gi)
-#pragma unroll
-        for (int m = 0; m < (1 << rl); ++m) {
-          const uint32_t v = mul_q(x[gi * (1 << rl) + m], n_inv);
-          buf[act_swz(tail_index<L>(gi * NT + g, m, s0l, rl))] =
-              (k < tg && bits * k < 32) ? (v >> (bits * k)) & mask : 0u;
-        }
-      __syncthreads();
-#pragma unroll
-      for (int b = 0; b < 8; ++b) x[b] = buf[act_swz(g + b * NT)];
+    *reinterpret_cast<uint4 *>(out) = make_uint4(x[0], x[1], x[2], x[3]);
+    out -= (size_t)C * n;
+    // after a timeout (recorded in *err) the walk goes on, so that every barrier of the block is met by all its threads
+    mbar_wait<true>(bar0 + 8 * pb, (uint32_t)phase, err, ALTO_ERR_WAIT_FULL, &bail);
+    const uint4 *p = reinterpret_cast<const uint4 *>(parts + (size_t)pb * C * n) + g;
+    uint4 u = p[0];
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+    for (int r = 1; r < C; ++r) {
+      u = p[r * (n / 4)];
+      x[0] = lazy_add(x[0], u.x); x[1] = lazy_add(x[1], u.y); x[2] = lazy_add(x[2], u.z); x[3] = lazy_add(x[3], u.w);
     }
-    fwd_round<L>(x, g, 3, 1, n >> 1, psi);
 #pragma unroll
-    for (int s0 = 3; s0 < L; s0 += 3) {
-      const int sr = (L - s0) < 3 ? (L - s0) : 3, t = n >> (s0 + 1), pt = n >> (s0 - 2);
-      uint32_t *buf = osm + (ex++ & 1) * n;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) buf[act_swz(fwd_pos<L>(g, 0, b, 3, pt))] = x[b];
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < 8 / (1 << sr); ++q)
-#pragma unroll
-        for (int b = 0; b < (1 << sr); ++b) x[q * (1 << sr) + b] = buf[act_swz(fwd_pos<L>(g, q, b, sr, t))];
-      fwd_round<L>(x, g, sr, 1 << s0, t, psi);
-    }
-    // bold_t[i][k], this CTA's share of the rotated sum, then the next r_i from every CTA's share
-    uint32_t *out = bt + (((size_t)chain * (half - 1) + i) * tg + k) * n;
-#pragma unroll
-    for (int q = 0; q < 8 / (1 << ls); ++q)
-#pragma unroll
-      for (int b = 0; b < (1 << ls); ++b) {
-        const int pos = fwd_pos<L>(g, q, b, ls, lt);
-        const uint32_t d = x[q * (1 << ls) + b];
-        if (k < tg) out[pos] = d;
-        const uint32_t v = k < tg ? mul_q(__ldg(w + k * n + auto_slot(e, pos, n, L)), d) : 0u;
-        for (int r = 0; r < C; ++r) cl.map_shared_rank(parts + ((size_t)pb * C + k) * n, r)[pos] = v;
-      }
-    cl.sync();  // every share has arrived in every CTA
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int sl = 8 * g + m;
-      uint32_t acc = mul_q(agg[m], n_inv);
-      for (int r = 0; r < C; ++r) acc = add_q(acc, parts[((size_t)pb * C + r) * n + sl]);
-      x[m] = acc;
-    }
+    for (int m = 0; m < 4; ++m) x[m] = canon_q(x[m]);
     pb ^= 1;
+    phase ^= pb ^ 1;  // each barrier's phases alternate
   }
-  cl.sync();  // no CTA exits while another may still write into its shared memory
+  cluster_sync_all();  // no CTA exits while another may still copy into its shared memory
   if (k == 0)
 #pragma unroll
-    for (int m = 0; m < 8; ++m) last[(size_t)chain * n + 8 * g + m] = x[m];
+    for (int m = 0; m < 4; ++m) last[(size_t)chain * n + 4 * g + m] = mul_q(x[m], n);
 }
 
 // Per output (one CTA each): bold_t_hat = NTT(G^-1(rbar_0)); a_hat = INTT(r_0 + sum_k v[k] bold_t_hat[k]).  Writes

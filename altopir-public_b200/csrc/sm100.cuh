@@ -40,25 +40,37 @@ __device__ __forceinline__ void fence_barrier_init() {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// CLUSTER: acquire what other CTAs of the cluster stored before their arrivals.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Waits for the phase with the given parity to complete.  Returns false (and ORs `code` into *err) after
 // ALTO_WAIT_NS of wall time, or at once when another role of this CTA has already recorded an error.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code,
                                           volatile int *bail) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
   const uint64_t t0 = globaltimer();
   for (uint32_t it = 0;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     if ((it & 63u) == 63u) {
       if (*bail) return false;
       if (globaltimer() - t0 > ALTO_WAIT_NS) {
@@ -216,6 +228,13 @@ __device__ __forceinline__ void cluster_sync_all() {
 // Arrive on an mbarrier given by its shared::cluster address (possibly in the peer CTA).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Copies `bytes` (a multiple of 16, 16-byte aligned) of this CTA's shared memory to another CTA's (a shared::cluster
+// address); their arrival counts as transaction bytes on that CTA's mbarrier.
+__device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "r"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 // TMA load into this CTA's shared memory whose completion is counted on the pair leader's mbarrier
 // (bar_cluster is a shared::cluster address).  No multicast: each CTA loads only its own tile.

@@ -1,0 +1,41 @@
+"""The arithmetic and the kernels of the offline set-up's register transforms."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "altopir-public_b200", "csrc")
+
+
+def test_montgomery_products_and_lazy_sums(tmp_path):
+    cxx = shutil.which("g++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path / "mont")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-I", CSRC, os.path.join(HERE, "cpp", "test_mont.cpp"), "-o", exe],
+                   check=True)
+    assert subprocess.run([exe], capture_output=True, text=True, timeout=300).stdout.strip() == "0"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tg", [2, 3, 5, 8])
+def test_register_walk_equals_the_single_cta_walk(gpu, svc, tg, monkeypatch):
+    """Clusters of 2, 3, 5 and 8 CTAs (one a digit): the walk with register transforms gives the values of the
+    single-CTA walk with shared-memory transforms, over a database of random bytes, all 255 and all zero columns."""
+    from altopir_b200 import offline
+    p = svc.Params(2048, 4096, tg=tg)
+    db = np.random.default_rng(tg).integers(0, 256, size=(p.record_bytes, p.rows), dtype=np.uint8)
+    db[::3] = 255
+    db[1::7] = 0
+    got = []
+    for variant in ({}, {"ALTO_OFFLINE_CLUSTER": "1", "ALTO_OFFLINE_ACT8": "0"}):
+        for k, v in variant.items():
+            monkeypatch.setenv(k, v)
+        e = offline.blank_engine(p, db)
+        got.append(offline.prepare(e, p, want=True)[1])
+        e.close()
+    for name in ("bold_t", "bold_t_bar", "that", "a_hat"):
+        assert np.array_equal(got[0][name], got[1][name]), name
