@@ -138,6 +138,27 @@ bool make_tile_map(CUtensorMap *m, const void *base, uint64_t kbs, uint64_t mts)
   return true;
 }
 
+// The same operand read in boxes of `rows` rows of `tiles` consecutive k blocks, without swizzling: [tile][row][128 bytes].
+bool make_rows_map(CUtensorMap *m, const void *base, uint64_t kbs, uint64_t mts, uint32_t rows, uint32_t tiles) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled is unavailable");
+    return false;
+  }
+  const cuuint64_t dims[4] = {128, 128, kbs, mts};
+  const cuuint64_t strides[3] = {128, 16384, 16384 * kbs};
+  const cuuint32_t box[4] = {128, rows, tiles, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed for the offline set-up's rows");
+    return false;
+  }
+  return true;
+}
+
 size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Uploads a row-major host matrix (nrows rows of k_bytes bytes, row pitch `pitch`) into the tile-contiguous layout
@@ -1851,7 +1872,7 @@ int alto_hint_ring(void *p, const uint64_t *query, uint64_t *out, int perm_out) 
   step(cudaMemcpy(d_psi_inv, psi_inv.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
   const unsigned threads = (unsigned)std::max<size_t>(32, std::min<size_t>(256, n / 2));
   if (err == cudaSuccess) {
-    alto::hint_query_kernel<<<(unsigned)polys, threads, n * sizeof(uint32_t)>>>(d_query, (int)n, d_psi, n_inv,
+    alto::hint_query_kernel<><<<(unsigned)polys, threads, n * sizeof(uint32_t)>>>(d_query, (int)n, d_psi, n_inv,
                                                                                d_qhat);
     step(cudaGetLastError());
   }
@@ -1963,29 +1984,21 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   step(cudaMemcpy(d_v, v32.data(), tg * n * sizeof(uint32_t), cudaMemcpyHostToDevice));
   step(cudaMemcpy(d_dlog, dlog.data(), n * sizeof(int16_t), cudaMemcpyHostToDevice));
   step(cudaMemcpy(d_inv_odd, inv_odd.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice));
-  const size_t act_smem = (1 + alto::kActCols) * n * sizeof(uint32_t), walk_smem = (1 + tg) * n * sizeof(uint32_t);
+  const size_t act_smem = (1 + alto::kActSmemCols) * n * sizeof(uint32_t), walk_smem = (1 + tg) * n * sizeof(uint32_t);
   step(cudaFuncSetAttribute(alto::offline_act_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)act_smem));
-  // n = 2048: the act kernel with register transforms (ALTO_OFFLINE_ACT8=0 runs the shared-memory one)
-  bool act8 = true;
-  if (const char *v = getenv("ALTO_OFFLINE_ACT8")) act8 = v[0] != '0';
-  // columns a CTA of the register-transform act kernel accumulates (ALTO_OFFLINE_ACTCOLS: 1, 2, 4 or 8).  Fewer
-  // columns keep less shared memory, so more CTAs share an SM: at 64 GiB the set-up took 736 ms with 8, 613 with 4,
-  // 586 with 2 and 582 with 1; at 1 GiB 31.4, 29.8, 29.4 and 29.5 ms.
-  int act_cols = 2;
-  if (const char *v = getenv("ALTO_OFFLINE_ACTCOLS")) {
-    const int c = atoi(v);
-    act_cols = c == 1 || c == 4 || c == 8 ? c : 2;
-  }
-  const size_t act8_smem = (2 + (size_t)act_cols) * n * sizeof(uint32_t);
-  if (n == 2048) {
-    step(cudaFuncSetAttribute(alto::offline_act8_kernel<11, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)((2 + 1) * n * sizeof(uint32_t))));
-    step(cudaFuncSetAttribute(alto::offline_act8_kernel<11, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)((2 + 2) * n * sizeof(uint32_t))));
-    step(cudaFuncSetAttribute(alto::offline_act8_kernel<11, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)((2 + 4) * n * sizeof(uint32_t))));
-    step(cudaFuncSetAttribute(alto::offline_act8_kernel<11, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)((2 + 8) * n * sizeof(uint32_t))));
+  // n = 2048: the hint on the tensor cores (ALTO_OFFLINE_ACT8=0 runs the shared-memory transforms)
+  bool act_mma = n == 2048;
+  if (const char *v = getenv("ALTO_OFFLINE_ACT8")) act_mma = act_mma && v[0] != '0';
+  uint8_t *d_dft = nullptr;
+  CUtensorMap map_rows, map_dft;
+  int sms = 148;
+  if (act_mma) {
+    step(cudaMalloc(&d_dft, alto::kActWBytes));
+    step(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
+    step(cudaFuncSetAttribute(alto::offline_act_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, alto::kActSmem));
+    if (err == cudaSuccess && (!make_rows_map(&map_rows, e->d_db, e->db_kbs, e->db_mts, alto::kActCols, 16) ||
+                               !make_map(&map_dft, d_dft, 128, 4 * 128, 128, 128)))
+      err = cudaErrorInvalidValue;
   }
   step(cudaFuncSetAttribute(alto::offline_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem));
   step(cudaFuncSetAttribute(alto::offline_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem));
@@ -2012,23 +2025,16 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   if (err == cudaSuccess) {
     step(cudaEventRecord(t0, 0));
     // the hint's query: NTT(perm(q_p)), without the n^-1 the coefficient-domain hint folds in
-    alto::hint_query_kernel<<<(unsigned)polys, nt, n * sizeof(uint32_t)>>>(d_q, (int)n, d_psi, 1u, d_qhat);
-    step(cudaGetLastError());
-    if (n == 2048 && act8 && act_cols == 1) {
-      alto::offline_act8_kernel<11, 1><<<(unsigned)cols, 256, act8_smem>>>(e->d_db, e->db_kbs, (int)polys, d_qhat,
-                                                                         d_psi, d_act);
-    } else if (n == 2048 && act8 && act_cols == 2) {
-      alto::offline_act8_kernel<11, 2><<<(unsigned)(cols / 2), 256, act8_smem>>>(e->d_db, e->db_kbs, (int)polys,
-                                                                               d_qhat, d_psi, d_act);
-    } else if (n == 2048 && act8 && act_cols == 4) {
-      alto::offline_act8_kernel<11, 4><<<(unsigned)(cols / 4), 256, act8_smem>>>(e->d_db, e->db_kbs, (int)polys,
-                                                                               d_qhat, d_psi, d_act);
-    } else if (n == 2048 && act8) {
-      alto::offline_act8_kernel<11, 8><<<(unsigned)(cols / 8), 256, act8_smem>>>(e->d_db, e->db_kbs, (int)polys,
-                                                                               d_qhat, d_psi, d_act);
+    if (act_mma) {
+      const int groups = (int)(cols / alto::kActCols);
+      alto::hint_query_kernel<true><<<(unsigned)polys, nt, n * sizeof(uint32_t)>>>(d_q, (int)n, d_psi, 1u, d_qhat);
+      alto::offline_dft_kernel<<<128, 128>>>(d_psi, d_dft);
+      alto::offline_act_mma_kernel<<<(unsigned)std::min(sms, groups), alto::kActThreads, alto::kActSmem>>>(
+          map_rows, map_dft, (int)polys, groups, reinterpret_cast<const uint4 *>(d_qhat), d_psi, d_act, e->main.d_err);
     } else {
-      alto::offline_act_kernel<<<(unsigned)(cols / alto::kActCols), 256, act_smem>>>(e->d_db, e->db_kbs, (int)n,
-                                                                                    (int)polys, d_qhat, d_psi, d_act);
+      alto::hint_query_kernel<><<<(unsigned)polys, nt, n * sizeof(uint32_t)>>>(d_q, (int)n, d_psi, 1u, d_qhat);
+      alto::offline_act_kernel<<<(unsigned)(cols / alto::kActSmemCols), 256, act_smem>>>(e->d_db, e->db_kbs, (int)n,
+                                                                                        (int)polys, d_qhat, d_psi, d_act);
     }
     step(cudaGetLastError());
     alto::offline_rows_kernel<<<(unsigned)cols, nt, n * sizeof(uint32_t)>>>(d_act, (int)n, d_psi);
@@ -2092,7 +2098,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   if (a_hat) step(cudaMemcpy(a_hat, d_ahat, outputs * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   for (void *x : {(void *)d_q, (void *)d_qhat, (void *)d_psi, (void *)d_psi_inv, (void *)d_w, (void *)d_v,
                   (void *)d_act, (void *)d_bt, (void *)d_last, (void *)d_dlog, (void *)d_inv_odd, (void *)d_that,
-                  (void *)d_ahat})
+                  (void *)d_ahat, (void *)d_dft})
     cudaFree(x);
   if (t0) cudaEventDestroy(t0);
   if (t1) cudaEventDestroy(t1);

@@ -40,7 +40,9 @@ __device__ __forceinline__ void hint_ntt_inv(uint32_t *a, int n, const uint32_t 
 }
 
 // The query's preprocessing, one CTA per polynomial: perm(q)[0] = q[0], perm(q)[i] = -q[n - i] (util.rs
-// negacyclic_perm with shift 0), then the forward transform, times n^-1.
+// negacyclic_perm with shift 0), then the forward transform, times n_inv.  BLOCKED stores slot 16 i + 4 v + u as word
+// 512 v + 4 i + u (n = 2048), the order in which offline_act_mma_kernel's threads read it.
+template <bool BLOCKED = false>
 __global__ void hint_query_kernel(const uint64_t *__restrict__ query, int n, const uint32_t *__restrict__ psi,
                                   uint32_t n_inv, uint32_t *__restrict__ qhat) {
   extern __shared__ uint32_t hsm[];
@@ -51,7 +53,8 @@ __global__ void hint_query_kernel(const uint64_t *__restrict__ query, int n, con
   }
   __syncthreads();
   hint_ntt_fwd(hsm, n, psi);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) qhat[(size_t)blockIdx.x * n + i] = mul_q(hsm[i], n_inv);
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    qhat[(size_t)blockIdx.x * n + (BLOCKED ? ((i >> 2) & 3) * 512 + (i >> 4) * 4 + (i & 3) : i)] = mul_q(hsm[i], n_inv);
 }
 
 // One CTA per database column `col`: acc = sum over its `polys` polynomials r of NTT(D_r) . qhat_r (pointwise), then

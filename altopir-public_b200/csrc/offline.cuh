@@ -32,7 +32,7 @@
 
 namespace alto {
 
-constexpr int kActCols = 8;  // database columns per CTA of the act kernel: 8 u32 = one 32-byte sector per slot
+constexpr int kActSmemCols = 8;  // database columns per CTA of the shared-memory act kernel: one 32-byte sector per slot
 
 __device__ __forceinline__ int brv_bits(int x, int logn) { return (int)(__brev((unsigned)x) >> (32 - logn)); }
 
@@ -79,7 +79,7 @@ __device__ __forceinline__ void digits_of(uint32_t *acc, uint32_t *dig, int n, i
   __syncthreads();
 }
 
-// act, one CTA per kActCols consecutive database columns: acc_c = sum_p NTT(D_(p,c)) . qhat_p (qhat = NTT(perm(q_p))),
+// act, one CTA per kActSmemCols consecutive database columns: acc_c = sum_p NTT(D_(p,c)) . qhat_p (qhat = NTT(perm(q_p))),
 // stored as actT[o][s][j] = acc_c[n - 1 - s] for column c = o n + j.  Database columns come from the engine's tile
 // layout as in hint_ring_kernel.
 __global__ void __launch_bounds__(256) offline_act_kernel(const uint8_t *__restrict__ db, size_t kbs, int n,
@@ -87,9 +87,9 @@ __global__ void __launch_bounds__(256) offline_act_kernel(const uint8_t *__restr
                                                           const uint32_t *__restrict__ psi, uint32_t *__restrict__ act) {
   extern __shared__ uint32_t osm[];
   uint32_t *a = osm, *acc = osm + n;
-  const size_t col0 = (size_t)blockIdx.x * kActCols;
-  for (int i = threadIdx.x; i < kActCols * n; i += blockDim.x) acc[i] = 0;
-  for (int c = 0; c < kActCols; ++c) {
+  const size_t col0 = (size_t)blockIdx.x * kActSmemCols;
+  for (int i = threadIdx.x; i < kActSmemCols * n; i += blockDim.x) acc[i] = 0;
+  for (int c = 0; c < kActSmemCols; ++c) {
     const size_t col = col0 + c;
     const uint8_t *row = db + (col / 128) * kbs * 16384 + (col % 128) * 128;
     for (int p = 0; p < polys; ++p) {
@@ -105,116 +105,254 @@ __global__ void __launch_bounds__(256) offline_act_kernel(const uint8_t *__restr
     }
   }
   __syncthreads();
-  const size_t o = col0 / n, j0 = col0 % n;  // kActCols divides n: the CTA's columns share their output
-  for (int idx = threadIdx.x; idx < n * kActCols; idx += blockDim.x) {
-    const int s = idx / kActCols, c = idx - s * kActCols;
+  const size_t o = col0 / n, j0 = col0 % n;  // kActSmemCols divides n: the CTA's columns share their output
+  for (int idx = threadIdx.x; idx < n * kActSmemCols; idx += blockDim.x) {
+    const int s = idx / kActSmemCols, c = idx - s * kActSmemCols;
     act[(o * n + s) * n + j0 + c] = acc[c * n + (n - 1 - s)];
   }
 }
 
-// Positions of a thread's 8 values in a round of s forward stages that starts at half-size t (n / 8 threads; each
-// holds 8 / 2^s groups of 2^s values): group grp = g + q n/8 is block blk = grp / d, offset r = grp % d, d = 2t / 2^s,
-// and its value b sits at blk 2t + r + b d.
-template <int L>
-__device__ __forceinline__ int fwd_pos(int g, int q, int b, int s, int t) {
-  const int G = 1 << s, d = 2 * t / G, grp = g + q * ((1 << L) / 8);
-  return (grp / d) * 2 * t + grp % d + b * d;
+// ------------------------------------------------------------------------------------ the hint on the tensor cores
+// acc_c = sum_p NTT(D_(p,c)) . qhat_p for n = 2048, the first seven of the transform's eleven stages as one byte-limb
+// product.  With index i = 16 j + r, block i' of 128 after those stages is the residue of D modulo X^16 - zeta_i',
+// zeta_i' = psi[128 + i']^2 (Cooley-Tukey stages over psi^brv), so its coefficient r is sum_j W[i'][j] x[16 j + r] with
+// W[i'][j] = zeta_i'^j: a 128 x 128 matrix of four byte limbs times the records' bytes, exact in int32 (128 x 255 x 255 <
+// 2^23).  A thread then holds the 16 coefficients of one block of one column, so the other four stages, the product with
+// qhat and the sum over p stay in its registers and nothing is exchanged.
+//
+// Operands.  A = the limbs of W, 128 rows x 128 bytes K-major with 128-byte swizzling, resident in shared memory.  B =
+// kActCols columns of the database for one p, N = (column, r), K = j: a tile row (one column, 128 records) holds eight j
+// of 16 r each, which is one 8 x 16-byte core matrix of an MN-major operand without swizzling; the next column is 128
+// bytes on (stride byte offset) and the next eight j the next tile (leading byte offset).  So the database tiles
+// are loaded as they are, 16 tiles x kActCols rows a box.  One accumulator of kActCols x 16 columns per limb, two
+// buffers: all of TMEM.
+//
+// Persistent, one CTA an SM: warps 0..15 transform (warp w: TMEM lanes 32 (w & 3).., column w >> 2), warp 16 loads, warp
+// 17 issues the MMAs.  Bound by the 16 warps' integer work (53 instructions a record byte, the multiplier pipe 78 %
+// busy; the tensor pipe 10 %).  Measured: 2.2 ms a GiB of database, against 8.9 with all eleven stages in registers and
+// one shared-memory exchange every three of them.
+constexpr int kActCols = 4;                            // database columns of a unit
+constexpr int kActStageBytes = 16 * kActCols * 128;    // one p of a unit: 16 tiles x kActCols rows
+constexpr int kActStages = 8;
+constexpr int kActWBytes = 4 * 128 * 128;
+constexpr int kActThreads = 18 * 32;
+constexpr int kActTwBytes = 15 * 128 * 4, kActOutBytes = 2048 * kActCols * 4;
+constexpr int kActSmem = 1024 + kActWBytes + kActStages * kActStageBytes + kActTwBytes + kActOutBytes + 256;
+
+// The byte limbs of W: w[(l 128 + i') 128 + j] = byte l of zeta_i'^j mod Q.
+__global__ void offline_dft_kernel(const uint32_t *__restrict__ psi, uint8_t *__restrict__ w) {
+  const int i = blockIdx.x, j = threadIdx.x;
+  uint32_t b = __ldg(psi + 128 + i), r = 1;
+  b = mul_q(b, b);
+  for (int k = j; k; k >>= 1) {
+    if (k & 1) r = mul_q(r, b);
+    b = mul_q(b, b);
+  }
+  for (int l = 0; l < 4; ++l) w[(l * 128 + i) * 128 + j] = (uint8_t)(r >> (8 * l));
 }
 
-// One round of s Cooley-Tukey stages (Longa-Naehrig Algorithm 1) on the thread's values: stage k of the round has
-// half-size t >> k and m << k blocks; its pairs are b, b + 2^(s-1-k) inside a group, twiddle psi[(m << k) + (blk << k) +
-// (b >> (s - k))].
-template <int L>
-__device__ __forceinline__ void fwd_round(uint32_t (&x)[8], int g, int s, int m, int t,
-                                          const uint32_t *__restrict__ psi) {
-  const int G = 1 << s, d = 2 * t / G;
-#pragma unroll
-  for (int q = 0; q < 8 / G; ++q) {
-    const int blk = (g + q * ((1 << L) / 8)) / d;
-#pragma unroll
-    for (int k = 0; k < s; ++k) {
-      const int half = G >> (k + 1);
-#pragma unroll
-      for (int b = 0; b < G; ++b) {
-        if (b & half) continue;
-        const uint32_t w = __ldg(psi + (m << k) + (blk << k) + (b >> (s - k)));
-        const uint32_t u = x[q * G + b], v = mul_q(x[q * G + b + half], w);
-        x[q * G + b] = add_q(u, v);
-        x[q * G + b + half] = sub_q(u, v);
-      }
-    }
-  }
+// (a0, a1, a2) += x y as a 96-bit sum
+__device__ __forceinline__ void mac96(uint32_t &a0, uint32_t &a1, uint32_t &a2, uint32_t x, uint32_t y) {
+  const uint64_t p = (uint64_t)x * y;
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
+      : "+r"(a0), "+r"(a1), "+r"(a2)
+      : "r"((uint32_t)p), "r"((uint32_t)(p >> 32)));
 }
 
-__device__ __forceinline__ int act_swz(int pos) { return pos ^ ((pos >> 5) & 31); }
+// Cooley-Tukey butterfly on 32-bit representatives (lazy_add), Gentleman-Sande on residues; twiddles in Montgomery form.
+__device__ __forceinline__ void bf_ct(uint32_t &x, uint32_t &y, uint32_t wm) {
+  const uint32_t v = mont_q(y, wm);
+  y = lazy_sub(x, v);
+  x = lazy_add(x, v);
+}
+__device__ __forceinline__ void bf_gs(uint32_t &x, uint32_t &y, uint32_t wm) {
+  const uint32_t s = add_q(x, y);
+  y = mont_q(sub_q(x, y), wm);
+  x = s;
+}
 
-// The act kernel with the transforms in registers: n / 8 threads, 8 values each, three stages per round and one
-// shared-memory exchange between rounds (double-buffered: one barrier an exchange), against a barrier per stage in
-// offline_act_kernel; ACOLS columns a CTA.  Same output.
-template <int L, int ACOLS>
-__global__ void __launch_bounds__((1 << L) / 8) offline_act8_kernel(const uint8_t *__restrict__ db, size_t kbs,
-                                                                     int polys, const uint32_t *__restrict__ qhat,
-                                                                     const uint32_t *__restrict__ psi,
-                                                                     uint32_t *__restrict__ act) {
-  constexpr int n = 1 << L, NT = n / 8;
-  static_assert(ACOLS >= 1 && n % ACOLS == 0, "columns per CTA");
-  extern __shared__ uint32_t osm[];
-  uint32_t *accs = osm + 2 * n;  // [column in CTA][position]
-  const int g = threadIdx.x;
-  const size_t col0 = (size_t)blockIdx.x * ACOLS;
-  int ex = 0;  // exchanges so far: buffer ex & 1
-  for (int c = 0; c < ACOLS; ++c) {
-    const size_t col = col0 + c;
-    const uint8_t *row = db + (col / 128) * kbs * 16384 + (col % 128) * 128;
-    uint32_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int p = 0; p < polys; ++p) {
-      uint32_t x[8];
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {  // the first round's positions: g + b n / 8
-        const size_t rec = (size_t)p * n + g + b * NT;
-        x[b] = row[(rec >> 7) * 16384 + (rec & 127)];
-      }
-#pragma unroll
-      for (int s0 = 0; s0 < L; s0 += 3) {
-        const int s = (L - s0) < 3 ? (L - s0) : 3, t = n >> (s0 + 1);
-        if (s0 > 0) {
-          const int ps = 3, pt = n >> (s0 - 3 + 1);  // every round before the last has three stages
-          uint32_t *buf = osm + (ex & 1) * n;
-#pragma unroll
-          for (int q = 0; q < 8 / (1 << ps); ++q)
-#pragma unroll
-            for (int b = 0; b < (1 << ps); ++b) buf[act_swz(fwd_pos<L>(g, q, b, ps, pt))] = x[q * (1 << ps) + b];
-          __syncthreads();
-#pragma unroll
-          for (int q = 0; q < 8 / (1 << s); ++q)
-#pragma unroll
-            for (int b = 0; b < (1 << s); ++b) x[q * (1 << s) + b] = buf[act_swz(fwd_pos<L>(g, q, b, s, t))];
-          ++ex;
-        }
-        fwd_round<L>(x, g, s, 1 << s0, t, psi);
-      }
-      constexpr int ls = (L % 3) ? (L % 3) : 3, lt = n >> (L - ls + 1);  // the last round
-      const uint32_t *qh = qhat + (size_t)p * n;
-#pragma unroll
-      for (int q = 0; q < 8 / (1 << ls); ++q)
-#pragma unroll
-        for (int b = 0; b < (1 << ls); ++b) {
-          const int i = q * (1 << ls) + b;
-          acc[i] = add_q(acc[i], mul_q(x[i], __ldg(qh + fwd_pos<L>(g, q, b, ls, lt))));
-        }
+// qhat in the order the transform threads read it: word (p 4 + v) 512 + 4 i' + u is slot 16 i' + 4 v + u (hint_query_kernel
+// with BLOCKED).  act[(o n + s) n + j] = acc_c[n - 1 - s], c = o n + j, as offline_act_kernel writes it.
+__global__ void __launch_bounds__(kActThreads, 1)
+    offline_act_mma_kernel(const __grid_constant__ CUtensorMap map_db, const __grid_constant__ CUtensorMap map_w,
+                           int polys, int groups, const uint4 *__restrict__ qhat, const uint32_t *__restrict__ psi,
+                           uint32_t *__restrict__ act, uint32_t *err) {
+  constexpr int n = 2048, N = 16 * kActCols;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+  uint8_t *smem = smem_raw + (base - raw);
+  const uint32_t ring = base + kActWBytes;
+  uint32_t *tw = reinterpret_cast<uint32_t *>(smem + kActWBytes + kActStages * kActStageBytes);
+  uint32_t *stage_out = tw + 15 * 128;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(stage_out + 2048 * kActCols);
+  const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kActStages, accf0 = empty0 + 8 * kActStages,
+                 acce0 = accf0 + 16, wbar = acce0 + 16;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kActStages + 5);
+  volatile int *bail = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < kActStages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
     }
-#pragma unroll
-    for (int q = 0; q < 8 / (1 << ((L % 3) ? (L % 3) : 3)); ++q) {
-      constexpr int ls = (L % 3) ? (L % 3) : 3, lt = n >> (L - ls + 1);
-#pragma unroll
-      for (int b = 0; b < (1 << ls); ++b) accs[c * n + fwd_pos<L>(g, q, b, ls, lt)] = acc[q * (1 << ls) + b];
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(accf0 + 8 * b, 1);
+      mbar_init(acce0 + 8 * b, 16);
     }
+    mbar_init(wbar, 1);
+    *bail = 0;
+    fence_barrier_init();
   }
+  if (warp == 16 && lane == 0) {
+    tma_prefetch_desc(&map_db);
+    tma_prefetch_desc(&map_w);
+  }
+  if (warp == 17) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  // twiddles of the last four stages, [stage and block][i']: psi[128 + i'], psi[256 + 2 i' + h], ...
+  for (int x = tid; x < 15 * 128; x += kActThreads) {
+    const int t = x >> 7, i = x & 127, st = t < 1 ? 0 : t < 3 ? 1 : t < 7 ? 2 : 3, h = t - ((1 << st) - 1);
+    tw[x] = to_mont(__ldg(psi + (128 << st) + (i << st) + h));
+  }
+  tc_fence_before();
   __syncthreads();
-  const size_t o = col0 / n, j0 = col0 % n;
-  for (int idx = threadIdx.x; idx < n * ACOLS; idx += NT) {
-    const int s = idx / ACOLS, c = idx - s * ACOLS;
-    act[(o * n + s) * n + j0 + c] = accs[c * n + (n - 1 - s)];
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  // Every wait is bounded; after a timeout (recorded in *err, with the bail flag) the later ones fail within a few polls, the
+  // loaders and the MMA issuer stop, and the transform warps run on to the end, so that they meet their barriers.
+  if (warp == 16) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(wbar, kActWBytes);
+      for (int l = 0; l < 4; ++l) tma_load_2d(base + l * 16384, &map_w, wbar, 0, 128 * l, policy_evict_normal());
+      const uint64_t pol = policy_evict_first();
+      int g = 0;
+      bool stop = false;
+      for (int u = blockIdx.x; u < groups && !stop; u += gridDim.x) {
+        const int col = u * kActCols, mt = col >> 7, row = col & 127;
+        for (int p = 0; p < polys; ++p, ++g) {
+          const int s = g % kActStages, round = g / kActStages;
+          if (round > 0 && !mbar_wait(empty0 + 8 * s, (round - 1) & 1, err, ALTO_ERR_WAIT_EMPTY, bail)) {
+            stop = true;
+            break;
+          }
+          mbar_arrive_expect_tx(full0 + 8 * s, kActStageBytes);
+          tma_load_rows(ring + s * kActStageBytes, &map_db, full0 + 8 * s, row, 16 * p, mt, pol);
+        }
+      }
+      if (stop) {  // loads already issued land within microseconds
+        const uint64_t t0 = globaltimer();
+        while (globaltimer() - t0 < 200000ull) {
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 17) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = idesc_u8u8_s32(N) | (1u << 16);  // B is MN-major
+      int g = 0;
+      bool stop = !mbar_wait(wbar, 0, err, ALTO_ERR_WAIT_FULL, bail);
+      for (int u = blockIdx.x; u < groups && !stop; u += gridDim.x) {
+        for (int p = 0; p < polys; ++p, ++g) {
+          const int s = g % kActStages, round = g / kActStages, b = g & 1, use = g >> 1;
+          if (use > 0 && !mbar_wait(acce0 + 8 * b, (use - 1) & 1, err, ALTO_ERR_WAIT_ACCUM, bail)) stop = true;
+          if (stop || !mbar_wait(full0 + 8 * s, round & 1, err, ALTO_ERR_WAIT_FULL, bail)) {
+            stop = true;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sb = ring + s * kActStageBytes;
+#pragma unroll
+          for (int l = 0; l < 4; ++l)
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)  // 32 j: four tiles
+              mma_i8(tmem + (uint32_t)((b * 4 + l) * N), desc_sw128(base + l * 16384 + kk * 32),
+                     desc_mn_plain(sb + kk * 4 * (kActCols * 128), kActCols * 128, 128), idesc, kk != 0);
+          mma_commit(empty0 + 8 * s);
+          mma_commit(accf0 + 8 * b);
+        }
+      }
+      if (*bail) {  // MMAs issued so far complete before TMEM and shared memory go away
+        const uint64_t t0 = globaltimer();
+        while (globaltimer() - t0 < 200000ull) {
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, c = warp >> 2, i = q * 32 + lane;  // block i' of column c
+    int g = 0;
+    for (int u = blockIdx.x; u < groups; u += gridDim.x) {
+      uint32_t a0[16], a1[16], a2[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a0[k] = a1[k] = a2[k] = 0;
+      for (int p = 0; p < polys; ++p, ++g) {
+        const int b = g & 1, use = g >> 1;
+        mbar_wait(accf0 + 8 * b, use & 1, err, ALTO_ERR_WAIT_ACCUM, bail);
+        tc_fence_after();
+        const uint32_t ta = tmem + (uint32_t)(b * 4 * N + 16 * c) + ((uint32_t)(q * 32) << 16);
+        uint32_t x[16];
+        {
+          uint32_t hi[16], lo[16];
+          tmem_ld16(ta + 2 * N, x);
+          tmem_ld16(ta + 3 * N, hi);
+          tmem_wait_ld();
+#pragma unroll
+          for (int k = 0; k < 16; ++k) x[k] += hi[k] << 8;  // < 2^32
+          tmem_ld16(ta, lo);
+          tmem_ld16(ta + N, hi);
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acce0 + 8 * b);
+          // lo + 2^8 hi + 2^16 x: the high half of x folds to 12287 (x >> 16) < 2^30, so that sum stays below 2^32 - 12287
+#pragma unroll
+          for (int k = 0; k < 16; ++k) x[k] = lazy_add(x[k] << 16, lo[k] + (hi[k] << 8) + (x[k] >> 16) * kFold);
+        }
+        const uint32_t *t = tw + i;
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+          const int h = 8 >> st;
+#pragma unroll
+          for (int blk = 0; blk < (1 << st); ++blk) {
+            const uint32_t wm = t[((1 << st) - 1 + blk) * 128];
+#pragma unroll
+            for (int r = 0; r < h; ++r) bf_ct(x[blk * 2 * h + r], x[blk * 2 * h + h + r], wm);
+          }
+        }
+        const uint4 *qp = qhat + (size_t)p * 512 + i;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const uint4 y = __ldg(qp + 128 * v);
+          mac96(a0[4 * v], a1[4 * v], a2[4 * v], x[4 * v], y.x);
+          mac96(a0[4 * v + 1], a1[4 * v + 1], a2[4 * v + 1], x[4 * v + 1], y.y);
+          mac96(a0[4 * v + 2], a1[4 * v + 2], a2[4 * v + 2], x[4 * v + 2], y.z);
+          mac96(a0[4 * v + 3], a1[4 * v + 3], a2[4 * v + 3], x[4 * v + 3], y.w);
+        }
+      }
+      // 2^32 = 12287 and 2^64 = 12287^2 (mod Q); a2 < 2^32 / 12287^2 products
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        stage_out[(k * 128 + i) * kActCols + c] =
+            red_q64((uint64_t)a1[k] * kFold + a0[k] + (uint64_t)a2[k] * ((uint64_t)kFold * kFold));
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      const size_t col = (size_t)u * kActCols, o = col / n, j0 = col % n;
+      for (int y = tid; y < 2048; y += 512) {
+        const int s = 16 * (y & 127) + (y >> 7);
+        *reinterpret_cast<uint4 *>(act + (o * n + (n - 1 - s)) * n + j0) =
+            *reinterpret_cast<const uint4 *>(stage_out + y * kActCols);
+      }
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 17) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
   }
 }
 
@@ -354,18 +492,6 @@ __device__ __forceinline__ void load_tw(RegTwiddles &t, const uint32_t *__restri
     t.a[q][1] = to_mont(__ldg(psi + 2 * base + 1));
   }
   t.d = to_mont(__ldg(psi + 1));
-}
-
-// Two butterflies each: Gentleman-Sande on residues, Cooley-Tukey on 32-bit representatives (lazy_add).
-__device__ __forceinline__ void bf_gs(uint32_t &x, uint32_t &y, uint32_t wm) {
-  const uint32_t s = add_q(x, y);
-  y = mont_q(sub_q(x, y), wm);
-  x = s;
-}
-__device__ __forceinline__ void bf_ct(uint32_t &x, uint32_t &y, uint32_t wm) {
-  const uint32_t v = mont_q(y, wm);
-  y = lazy_sub(x, v);
-  x = lazy_add(x, v);
 }
 
 __device__ __forceinline__ int swz4(int i) { return i ^ (((i >> 5) & 1) << 2) ^ (((i >> 6) & 1) * 0x18); }

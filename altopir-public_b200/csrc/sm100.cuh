@@ -115,6 +115,15 @@ __device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap *m
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"(kb), "r"(mt), "l"(cache_hint)
       : "memory");
 }
+// 4-D load of a few rows of consecutive tiles: coordinates (0, first row in the tile, first k block, 128-row tile).
+__device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t row, int32_t kb,
+                                              int32_t mt, uint64_t cache_hint) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2], %7;" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"(row), "r"(kb), "r"(mt), "l"(cache_hint)
+      : "memory");
+}
 // L2 cache policies for the loads (createpolicy fractions of 1.0).
 __device__ __forceinline__ uint64_t policy_evict_first() {
   uint64_t p;
@@ -158,6 +167,13 @@ __device__ __forceinline__ void tc_fence_after() {
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
   return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) |
          ((uint64_t)1u << 46) | ((uint64_t)2u << 61);
+}
+
+// Shared-memory matrix descriptor of an MN-major operand without swizzling: core matrices of 8 (K) x 16 bytes (M or N), 128
+// bytes each, the next 16 along M or N at `stride` bytes and the next 8 along K at `leading` bytes.  Layout type 0.
+__device__ __forceinline__ uint64_t desc_mn_plain(uint32_t smem_addr, uint32_t leading, uint32_t stride) {
+  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)(leading >> 4) << 16) | ((uint64_t)(stride >> 4) << 32) |
+         ((uint64_t)1u << 46);
 }
 
 // Instruction descriptor of tcgen05.mma kind::i8 with unsigned 8-bit A and B (both K-major), signed 32-bit
@@ -224,6 +240,10 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrive on an mbarrier of this CTA.
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Arrive on an mbarrier given by its shared::cluster address (possibly in the peer CTA).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {

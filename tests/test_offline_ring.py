@@ -21,12 +21,14 @@ def test_montgomery_products_and_lazy_sums(tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tg", [2, 3, 5, 8])
-def test_register_walk_equals_the_single_cta_walk(gpu, svc, tg, monkeypatch):
-    """Clusters of 2, 3, 5 and 8 CTAs (one a digit): the walk with register transforms gives the values of the
-    single-CTA walk with shared-memory transforms, over a database of random bytes, all 255 and all zero columns."""
+@pytest.mark.parametrize("rows,record,tg", [(2048, 2048, 2), (2048, 4096, 3), (2048 * 9, 4096, 5), (2048 * 20, 6144, 8)])
+def test_register_transforms_equal_the_shared_memory_ones(gpu, svc, rows, record, tg, monkeypatch):
+    """The hint on the tensor cores and the walk with register transforms on clusters of 2, 3, 5 and 8 CTAs (one a digit)
+    give the values of the shared-memory transforms and the single-CTA walk, over a database of random bytes, all 255
+    and all zero columns: from one polynomial a column to more than the loader's stages, and from fewer column groups
+    than four an SM to a partial last round."""
     from altopir_b200 import offline
-    p = svc.Params(2048, 4096, tg=tg)
+    p = svc.Params(rows, record, tg=tg)
     db = np.random.default_rng(tg).integers(0, 256, size=(p.record_bytes, p.rows), dtype=np.uint8)
     db[::3] = 255
     db[1::7] = 0
