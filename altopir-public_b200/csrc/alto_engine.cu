@@ -1917,27 +1917,8 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   while ((size_t(1) << logn) < n) ++logn;
   // gadget digits: floor(32 / t) + 1 bits each (one bit when t = 32), as get_bits_per gives for log2ceil(Q) = 32
   const int bits = tg >= 32 ? 1 : (int)(32 / tg) + 1;
-  // dlog[(t - 1) / 2] = 2 i + bar for t = g^i (bar 0) or 2n - g^i (bar 1); inv_odd[x] = (2x + 1)^-1 mod 2n
-  std::vector<int16_t> dlog(n, -1);
-  std::vector<uint16_t> inv_odd(n);
-  for (size_t i = 0, g = 1; i < half; ++i, g = (g * 5) % (2 * n)) {
-    dlog[(g - 1) / 2] = (int16_t)(2 * i);
-    dlog[(2 * n - g - 1) / 2] = (int16_t)(2 * i + 1);
-  }
-  for (size_t x = 0; x < n; ++x) {
-    // Newton's iteration for an odd a modulo a power of two: a a = 1 (mod 8), and inv (2 - a inv) doubles the bits that
-    // are right, so two steps give the 12 bits 2n needs (a^(n-1) by n - 2 multiplications took 23 ms a set-up at
-    // n = 2048, more than its largest kernel)
-    const uint32_t a = (uint32_t)(2 * x + 1);
-    uint32_t inv = a;
-    for (int k = 0; k < 2; ++k) inv *= 2u - a * inv;
-    inv_odd[x] = (uint16_t)(inv & (2 * n - 1));
-  }
-  for (size_t x = 0; x < n; ++x)
-    if (dlog[x] < 0 || (2 * x + 1) * inv_odd[x] % (2 * n) != 1) {
-      set_error("alto_engine_offline: automorphism tables");
-      return -1;
-    }
+  std::vector<uint16_t> gen(half);  // g^i mod 2n, g = 5
+  for (size_t i = 0, g = 1; i < half; ++i, g = (g * 5) % (2 * n)) gen[i] = (uint16_t)g;
   if (cudaSetDevice(e->dev) != cudaSuccess) return -4;
   for (int k = 0; k < e->lanes_made; ++k) {  // batches already enqueued read the packing state
     if (cudaStreamSynchronize(lane_batch(e, k)->st) != cudaSuccess ||
@@ -1955,8 +1936,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   uint64_t *d_q = nullptr;
   uint32_t *d_qhat = nullptr, *d_psi = nullptr, *d_psi_inv = nullptr, *d_w = nullptr, *d_v = nullptr;
   uint32_t *d_act = nullptr, *d_bt = nullptr, *d_last = nullptr, *d_that = nullptr, *d_ahat = nullptr;
-  int16_t *d_dlog = nullptr;
-  uint16_t *d_inv_odd = nullptr;
+  uint16_t *d_gen = nullptr;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   cudaError_t err = cudaSuccess;
   auto step = [&](cudaError_t x) {
@@ -1973,8 +1953,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   step(cudaMalloc(&d_act, cols * n * sizeof(uint32_t)));
   step(cudaMalloc(&d_bt, bt_words * sizeof(uint32_t)));
   step(cudaMalloc(&d_last, outputs * 2 * n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_dlog, n * sizeof(int16_t)));
-  step(cudaMalloc(&d_inv_odd, n * sizeof(uint16_t)));
+  step(cudaMalloc(&d_gen, half * sizeof(uint16_t)));
   if (that) step(cudaMalloc(&d_that, outputs * tg * n * sizeof(uint32_t)));
   if (a_hat) step(cudaMalloc(&d_ahat, outputs * n * sizeof(uint32_t)));
   step(cudaMemcpy(d_q, query, e->rows * sizeof(uint64_t), cudaMemcpyHostToDevice));
@@ -1982,8 +1961,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   step(cudaMemcpy(d_psi_inv, psi_inv.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
   step(cudaMemcpy(d_w, w32.data(), tg * n * sizeof(uint32_t), cudaMemcpyHostToDevice));
   step(cudaMemcpy(d_v, v32.data(), tg * n * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_dlog, dlog.data(), n * sizeof(int16_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_inv_odd, inv_odd.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice));
+  step(cudaMemcpy(d_gen, gen.data(), half * sizeof(uint16_t), cudaMemcpyHostToDevice));
   const size_t act_smem = (1 + alto::kActSmemCols) * n * sizeof(uint32_t), walk_smem = (1 + tg) * n * sizeof(uint32_t);
   step(cudaFuncSetAttribute(alto::offline_act_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)act_smem));
   // n = 2048: the hint on the tensor cores (ALTO_OFFLINE_ACT8=0 runs the shared-memory transforms)
@@ -1992,9 +1970,9 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   uint8_t *d_dft = nullptr;
   CUtensorMap map_rows, map_dft;
   int sms = 148;
+  step(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
   if (act_mma) {
     step(cudaMalloc(&d_dft, alto::kActWBytes));
-    step(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
     step(cudaFuncSetAttribute(alto::offline_act_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, alto::kActSmem));
     if (err == cudaSuccess && (!make_rows_map(&map_rows, e->d_db, e->db_kbs, e->db_mts, alto::kActCols, 16) ||
                                !make_map(&map_dft, d_dft, 128, 4 * 128, 128, 128)))
@@ -2021,7 +1999,8 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   // walk and finish threads: at least n / 4 (the cluster walk gathers 4 slots a thread ahead), at most 1024
   const unsigned wt = (unsigned)std::max<size_t>(std::max<size_t>(64, n / 4), std::min<size_t>(1024, tg * n / 2));
   const uint32_t tail_scale = alto::inv_pow2_q(logn);
-  const size_t K = tg * n, planes_threads = cols * K;
+  const size_t plane_smem = alto::kPlaneCols * (n + 4) * sizeof(uint32_t);
+  step(cudaFuncSetAttribute(alto::offline_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem));
   if (err == cudaSuccess) {
     step(cudaEventRecord(t0, 0));
     // the hint's query: NTT(perm(q_p)), without the n^-1 the coefficient-domain hint folds in
@@ -2037,7 +2016,10 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
                                                                                         (int)polys, d_qhat, d_psi, d_act);
     }
     step(cudaGetLastError());
-    alto::offline_rows_kernel<<<(unsigned)cols, nt, n * sizeof(uint32_t)>>>(d_act, (int)n, d_psi);
+    if (n == 2048)
+      alto::offline_rows8_kernel<<<(unsigned)std::min<size_t>(cols, 2 * (size_t)sms), 512>>>(d_act, (int)cols, d_psi);
+    else
+      alto::offline_rows_kernel<<<(unsigned)cols, nt, n * sizeof(uint32_t)>>>(d_act, (int)n, d_psi);
     step(cudaGetLastError());
     if (cluster > 1) {
       // one cluster of `cluster` CTAs per (output, chain), the digits split between them
@@ -2073,8 +2055,8 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
                                                                       d_psi_inv, n_inv, tail_scale, e->d_that,
                                                                       e->d_prefix, e->part_len, q2_bits, d_that, d_ahat);
     step(cudaGetLastError());
-    alto::offline_planes_kernel<<<(unsigned)((planes_threads + 255) / 256), 256>>>(
-        d_bt, (int)n, logn, (int)tg, cols, d_dlog, d_inv_odd, tail_scale, e->d_ub, e->ub_kbs);
+    alto::offline_planes_kernel<<<dim3((unsigned)(cols / alto::kPlaneCols), (unsigned)tg), 256, plane_smem>>>(
+        d_bt, (int)n, logn, (int)tg, d_gen, tail_scale, e->d_ub, e->ub_kbs);
     step(cudaGetLastError());
     // the engine's tail twiddles: its inverse table psi^-brv / 2, doubled as create_engine stores it
     step(cudaMemcpyAsync(e->d_tw, d_psi_inv, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, 0));
@@ -2097,7 +2079,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   if (that) step(cudaMemcpy(that, d_that, outputs * tg * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   if (a_hat) step(cudaMemcpy(a_hat, d_ahat, outputs * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   for (void *x : {(void *)d_q, (void *)d_qhat, (void *)d_psi, (void *)d_psi_inv, (void *)d_w, (void *)d_v,
-                  (void *)d_act, (void *)d_bt, (void *)d_last, (void *)d_dlog, (void *)d_inv_odd, (void *)d_that,
+                  (void *)d_act, (void *)d_bt, (void *)d_last, (void *)d_gen, (void *)d_that,
                   (void *)d_ahat, (void *)d_dft})
     cudaFree(x);
   if (t0) cudaEventDestroy(t0);

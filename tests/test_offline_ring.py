@@ -41,3 +41,27 @@ def test_register_transforms_equal_the_shared_memory_ones(gpu, svc, rows, record
         e.close()
     for name in ("bold_t", "bold_t_bar", "that", "a_hat"):
         assert np.array_equal(got[0][name], got[1][name]), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,tg", [(32, 4), (64, 8), (256, 4), (1024, 2)])
+def test_packing_matrix_at_other_ring_dimensions(gpu, oracle, svc, n, tg):
+    """Rings of 32 (several digits in one 128-byte tile row) to 1,024: the walk's values equal the oracle's, and the
+    responses, which read every byte of the packing matrix, too."""
+    from altopir_b200 import offline
+    from oracle.scheme import SchemeState
+    p = svc.Params(2 * n if n > 32 else 64, n, n=n, tg=tg)
+    db = np.random.default_rng(n).integers(0, 256, size=(p.record_bytes, p.rows), dtype=np.uint8)
+    st = SchemeState(p, db, oracle)
+    e = offline.blank_engine(p, db)
+    _, out = offline.prepare(e, p, want=True)
+    for k in ("bold_t", "bold_t_bar", "that"):
+        assert np.array_equal(out[k][0].astype(np.uint64), getattr(st, k)[0]), k
+    req = svc.synthetic_requests(p, 3, seed=n)
+    frames = [req[i] for i in range(3)]
+    _, _, want = oracle.answer(st, frames)
+    got = np.zeros((3, e.response_len()), dtype=np.uint8)
+    status = np.full(3, -1, dtype=np.int32)
+    assert e.answer(frames, got, status)[0] == 3
+    assert np.array_equal(got, want)
+    e.close()
