@@ -520,24 +520,26 @@ bool dispatch_gemm(int bn, const CUtensorMap &a, const CUtensorMap &b, const alt
   return false;
 }
 
-template <int BN, alto::Epi EPI, int NSUB = 1>
+template <int BN, alto::Epi EPI>
 bool launch_pair(const CUtensorMap &a, const CUtensorMap &b, const alto::PairArgs &g, int pairs, cudaStream_t st) {
-  const int smem = alto::PairShape<BN, NSUB>::kSmemBytes;
-  ALTO_CK(cudaFuncSetAttribute(alto::limb_gemm_pair_kernel<BN, EPI, NSUB>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  alto::limb_gemm_pair_kernel<BN, EPI, NSUB><<<2 * pairs, alto::kGemmThreads, smem, st>>>(a, b, g);
+  const int smem = alto::PairShape<BN>::kSmemBytes;
+  ALTO_CK(cudaFuncSetAttribute(alto::limb_gemm_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  alto::limb_gemm_pair_kernel<BN, EPI><<<2 * pairs, alto::kGemmThreads, smem, st>>>(a, b, g);
   ALTO_CK(cudaGetLastError());
   return true;
 }
 
-// bn = columns per accumulator; wide = two 256-column accumulators per unit (NSUB = 2, scan only)
+// bn = columns per accumulator; wide = units of two sub-accumulators of g.nw columns
 template <alto::Epi EPI>
 bool dispatch_pair(int bn, const CUtensorMap &a, const CUtensorMap &b, const alto::PairArgs &g, int pairs,
                    cudaStream_t st, bool wide = false) {
   if (wide) {
-    if (bn == 256) return launch_pair<256, EPI, 2>(a, b, g, pairs, st);
-    set_error("wide pair GEMM needs 256-column accumulators");
-    return false;
+    ALTO_CK(cudaFuncSetAttribute(alto::limb_gemm_wide_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 alto::kWideSmem));
+    alto::limb_gemm_wide_kernel<EPI><<<2 * pairs, alto::kWideThreads, alto::kWideSmem, st>>>(a, b, g,
+                                                                                            alto::wide_stages(g.nw));
+    ALTO_CK(cudaGetLastError());
+    return true;
   }
   switch (bn) {
     case 32: return launch_pair<32, EPI>(a, b, g, pairs, st);
@@ -581,16 +583,22 @@ int pick_bn(size_t limb_cols) {
   return 256;
 }
 
+// What a unit of a scan costs besides its blocks of K, in blocks (split_cost): measured at 1 GiB and 128 clients by units of
+// 19 to 86 blocks, 3.4 for wide units of 512 columns.
+constexpr double kWideExtra = 3.4, kTileExtra = 6;
+
 struct Plan {
   bool pair = false;  // CTA-pair kernels (limb columns > 16) or the single-CTA kernels
-  bool wide = false;  // scan units of 512 limb columns (one read of each database tile for all of them)
-  bool pack_wide = false;  // pack units of 512 limb columns (one read of each packing-matrix tile for all of them)
-  int scan_n = 1;     // scan tiles along the limb columns (num_n / 2 when wide)
+  bool wide = false;  // scan in wide units (one read of each database tile for up to 512 limb columns)
+  bool pack_wide = false;  // pack in wide units
+  int wide_nw = 0, wide_n = 0;  // a wide unit is 2 x wide_nw limb columns; wide_n units cover the batch
+  int scan_n = 1;     // scan units along the limb columns
   int kb_chunk = 1;   // scan blocks per record chunk
   int bn = 16, num_n = 1;
   int nw = 16;        // limb columns a pair-kernel tile computes: a multiple of 32 <= bn (bn: the kernel's template
                       // width, a power of two), num_n tiles covering the batch's limb columns with least padding
   int scan_m = 0, scan_split = 1, scan_kb_per = 1, scan_kb = 0;
+  bool split_each = false;  // every scan launch chooses its own blocks per unit (split_cost) instead of scan_kb_per
   int pack_m = 0, pack_kb = 0;
   int pairs_scan = 0, pairs_pack = 0;  // persistent grid of the pair kernels
 };
@@ -599,6 +607,32 @@ struct Plan {
 bool pair_kernels_enabled() {
   const char *v = getenv("ALTO_GEMM");
   return !(v && strcmp(v, "single") == 0);
+}
+
+// The persistent pairs take a launch's units, all of one length, in rounds, so it takes ceil(units / pairs) rounds of a
+// unit's blocks of K plus what a unit costs besides (its epilogue's reductions, the pipeline's refill), `extra` blocks.
+// Finds the split of `kb` blocks over `tiles` tiles with the least sum: returns it in blocks, its blocks per unit in *per.
+// 64 tiles of 256 blocks on 74 pairs (half of a 1 GiB scan, 128 clients): 8 units a tile make 7 rounds of 32 blocks, where
+// twelve units a pair made 7 units a tile, 7 rounds of 37.
+double split_cost(const Engine *e, int kb_chunk, long tiles, int kb, double extra, int *per) {
+  const int pairs = resident_pairs();
+  double cost = 0;
+  *per = 0;
+  auto look = [&](int p) {
+    const long units = tiles * ((kb + p - 1) / p), rounds = (units + pairs - 1) / pairs;
+    const double c = (double)rounds * (std::min(p, kb) + extra);
+    if (!*per || c < cost) {
+      *per = p;
+      cost = c;
+    }
+  };
+  if (e->nchunks > 1) {  // a unit's blocks divide a record chunk's 256
+    for (int p = kb_chunk; p >= 8; p /= 2) look(p);
+  } else {
+    const int least = (kb + 255) / 256;
+    for (int split = least; split == least || kb / split >= 8; ++split) look((kb + split - 1) / split);
+  }
+  return cost;
 }
 
 // The record-axis split is chosen for the whole scan; a scan run in column groups launches each group's share of
@@ -639,9 +673,9 @@ Plan make_plan(const Engine *e, size_t slots) {
   // (the pair kind::i8 MMA's N), as few tiles as the cap allows, each as narrow as covers the batch.  Narrow tiles are
   // taken when they cut the columns computed by at least 20 %, which leaves out 224-column tiles.  Measured at 8 GiB
   // (scan ms, power-of-two / narrow): 36 clients 1.83 / 1.54 on one 160-column tile (1.60 on 192); 48 clients
-  // 1.82 / 1.66 on 192; 136 clients 6.13 / 4.63 on 3 x 192; 70 clients 2.81 / 2.92 on 2 x 160 (the one loss);
-  // 224-column tiles (100 or 200 clients) ran 10-11 % slower than 256-column ones.  ALTO_TILE_EXACT=0 never takes
-  // narrow tiles, =1 always; ALTO_TILE_ALIGN=64 rounds their width to a multiple of 64.
+  // 1.82 / 1.66 on 192.  Several tiles are what batches of more than 256 limb columns take where wide units (below) are
+  // too few for the pairs.  ALTO_TILE_EXACT=0 never takes narrow tiles, =1 always; ALTO_TILE_ALIGN=64 rounds their width
+  // to a multiple of 64.
   {
     int bn2 = 32;
     while (bn2 < bn_cap && (size_t)bn2 < limb_cols) bn2 *= 2;
@@ -665,13 +699,28 @@ Plan make_plan(const Engine *e, size_t slots) {
   p.scan_m = (int)((e->cols + 255) / 256);
   p.pack_m = (int)((4 * e->cols + 255) / 256);
   const int pairs = resident_pairs();
-  // Wide scan units once the database spans several record chunks (its tiles then stream from HBM and cannot be
-  // shared between two pairs through L2) and there are at least 512 limb columns; ALTO_SCAN_WIDE=0/1 overrides.
-  const bool full = p.bn == 256 && p.nw == 256;  // wide units take two full 256-column sub-accumulators
-  p.wide = full && p.num_n >= 2 && e->nchunks > 1;
-  if (tn && tn->wide >= 0) p.wide = full && p.num_n >= 2 && tn->wide == 1;
-  if (const char *w = getenv("ALTO_SCAN_WIDE")) p.wide = full && p.num_n >= 2 && w[0] == '1';
-  p.scan_n = p.wide ? (p.num_n + 1) / 2 : p.num_n;
+  // More than 256 limb columns: wide units (two sub-accumulators, each A tile loaded once for both) or units of one
+  // tile, whichever makes the launch shorter by rounds of units (split_cost) times the cycles of a block of K: 4 nw + 180
+  // for a wide one of 2 nw columns, 2 nw + 100 for a tile of nw (the pack of 32 KB records, 448 blocks a pair: 541,000
+  // cycles at 2 x 256 columns, 364,000 at 2 x 160; 274,000 for a tile of 256).  Wide units win wherever there are enough
+  // of them: us a call, tiles / wide, 1 GiB 128 clients 995 / 942, 8 GiB 128 clients 4,570 / 3,900, 200 clients 8,200 /
+  // 6,700, 1024 clients 35,700 / 29,900.  ALTO_SCAN_WIDE and ALTO_PACK_WIDE = 0 / 1 override.
+  const bool can = bn_cap == 256 && limb_cols > 256;
+  p.split_each = limb_cols > 256 && !(tn && tn->units_per_pair > 0);
+  if (can) {
+    p.wide_n = (int)((limb_cols + 511) / 512);
+    p.wide_nw = (int)round_up((limb_cols + 2 * p.wide_n - 1) / (2 * p.wide_n), 32);
+    const double block_w = 4.0 * p.wide_nw + 180, block_n = 2.0 * p.nw + 100;
+    int per;
+    p.wide = split_cost(e, p.kb_chunk, (long)p.scan_m * p.wide_n, p.scan_kb, kWideExtra, &per) * block_w <=
+             split_cost(e, p.kb_chunk, (long)p.scan_m * p.num_n, p.scan_kb, kTileExtra, &per) * block_n;
+    auto rounds = [&](long units) { return (double)((units + pairs - 1) / pairs); };
+    p.pack_wide = rounds((long)p.pack_m * p.wide_n) * block_w <= rounds((long)p.pack_m * p.num_n) * block_n;
+  }
+  if (tn && tn->wide >= 0) p.wide = can && tn->wide == 1;
+  if (const char *w = getenv("ALTO_SCAN_WIDE")) p.wide = can && w[0] == '1';
+  if (const char *w = getenv("ALTO_PACK_WIDE")) p.pack_wide = can && w[0] == '1';
+  p.scan_n = p.wide ? p.wide_n : p.num_n;
   // Scan chunks: at most 256 blocks (exactness, as above), at least 8, and about twelve units per resident pair so
   // the persistent pairs finish together.
   const long tiles = (long)p.scan_m * p.scan_n;
@@ -681,11 +730,8 @@ Plan make_plan(const Engine *e, size_t slots) {
   split = std::max<long>(split, (p.scan_kb + 255) / 256);
   p.scan_kb_per = chunk_aligned((int)((p.scan_kb + split - 1) / split));
   p.scan_split = (p.scan_kb + p.scan_kb_per - 1) / p.scan_kb_per;
-  p.pairs_scan = (int)std::min<long>(pairs, tiles * p.scan_split);
-  // Wide pack units (ALTO_PACK_WIDE=1): both 256-column tiles of the limb columns in one unit, so each packing-
-  // matrix tile is read once (and the epilogue no longer overlaps the next unit's MMAs)
-  if (const char *w = getenv("ALTO_PACK_WIDE")) p.pack_wide = full && p.num_n >= 2 && w[0] == '1';
-  const long pack_n = p.pack_wide ? (p.num_n + 1) / 2 : p.num_n;
+  p.pairs_scan = pairs;  // at most one per unit of a launch
+  const long pack_n = p.pack_wide ? p.wide_n : p.num_n;
   p.pairs_pack = (int)std::min<long>(pairs, (long)p.pack_m * pack_n);
   return p;
 }
@@ -697,7 +743,10 @@ bool launch_scan(const Engine *e, const Plan &p, const CUtensorMap &map_q, uint3
   // (all records by default; a range starts and ends on record-chunk boundaries, so units never straddle one)
   if (mg < 0) mg = p.scan_m;
   if (kb_hi < 0) kb_hi = p.scan_kb;
-  const int splits = (kb_hi - kb_lo + p.scan_kb_per - 1) / p.scan_kb_per;
+  int kb_per = p.scan_kb_per;
+  if (p.split_each)
+    split_cost(e, p.kb_chunk, (long)mg * p.scan_n, kb_hi - kb_lo, p.wide ? kWideExtra : kTileExtra, &kb_per);
+  const int splits = (kb_hi - kb_lo + kb_per - 1) / kb_per;
   // The query limbs are re-read by every unit of a K chunk; mark them evict-last only while the whole operand
   // (4 bytes per record and client) is a small part of the 126 MB L2, so stale chunks never crowd it out.
   const int keep_b = 4 * round_up(slots, 4) * e->rows <= (size_t(32) << 20);
@@ -709,7 +758,7 @@ bool launch_scan(const Engine *e, const Plan &p, const CUtensorMap &map_q, uint3
     g.num_units = mg * p.scan_n * splits;
     g.kb_total = kb_hi;
     g.kb_begin = kb_lo;
-    g.kb_per_unit = p.scan_kb_per;
+    g.kb_per_unit = kb_per;
     g.rows_a = (int)e->cols;
     g.clients = (int)slots;
     g.cols = (int)e->cols;
@@ -717,7 +766,7 @@ bool launch_scan(const Engine *e, const Plan &p, const CUtensorMap &map_q, uint3
     g.err = err;
     g.b_keep = keep_b;
     g.kb_chunk = p.kb_chunk;
-    g.nw = p.nw;
+    g.nw = p.wide ? p.wide_nw : p.nw;
     return dispatch_pair<alto::Epi::kScan>(p.bn, e->map_db, map_q, g,
                                            std::min(p.pairs_scan, g.num_units), st, p.wide);
   }
@@ -745,7 +794,7 @@ bool launch_pack(const Engine *e, const Plan &p, const CUtensorMap &map_y, uint3
     alto::PairArgs g;
     g.num_m = p.pack_m;
     g.m_begin = 0;
-    g.num_n = p.pack_wide ? (p.num_n + 1) / 2 : p.num_n;
+    g.num_n = p.pack_wide ? p.wide_n : p.num_n;
     g.num_units = p.pack_m * g.num_n;
     g.kb_total = p.pack_kb;
     g.kb_per_unit = p.pack_kb;
@@ -756,7 +805,7 @@ bool launch_pack(const Engine *e, const Plan &p, const CUtensorMap &map_y, uint3
     g.err = err;
     g.b_keep = keep_b;
     g.kb_chunk = 1;
-    g.nw = p.nw;
+    g.nw = p.pack_wide ? p.wide_nw : p.nw;
     return dispatch_pair<alto::Epi::kPack>(p.bn, e->map_ub, map_y, g, p.pairs_pack, st, p.pack_wide);
   }
   alto::GemmArgs g;
@@ -779,9 +828,10 @@ bool launch_pack(const Engine *e, const Plan &p, const CUtensorMap &map_y, uint3
 // one half of a tile per CTA, for the pair kernels).
 bool make_limb_maps(const Engine *e, const Plan &p, const uint8_t *qlimb, const uint8_t *ylimb, size_t bp,
                     CUtensorMap *map_q, CUtensorMap *map_y) {
-  const uint32_t box = (uint32_t)(p.pair ? p.nw / 2 : p.bn);
-  return make_map3(map_q, qlimb, e->chunk, 4 * (uint64_t)bp, e->nchunks, box) &&
-         make_map(map_y, ylimb, e->count, 4 * (uint64_t)bp, e->count, box);
+  const uint32_t box_q = (uint32_t)(!p.pair ? p.bn : (p.wide ? p.wide_nw : p.nw) / 2);
+  const uint32_t box_y = (uint32_t)(!p.pair ? p.bn : (p.pack_wide ? p.wide_nw : p.nw) / 2);
+  return make_map3(map_q, qlimb, e->chunk, 4 * (uint64_t)bp, e->nchunks, box_q) &&
+         make_map(map_y, ylimb, e->count, 4 * (uint64_t)bp, e->count, box_y);
 }
 
 // Column groups of the scan and tail: group g is the response parts [bounds[g], bounds[g + 1]), whose columns are

@@ -121,49 +121,60 @@ __global__ void __launch_bounds__(kGemmThreads, GemmShape<BN>::kCtasPerSm)
   volatile int no_bail = 0;
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      // The A operand (database or packing matrix) streams through once per unit; B (limbs) is shared by all units.
-      const uint64_t pol_a = policy_evict_first();
-      const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
-      int issued = 0;
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % kStages, round = i / kStages;
-        if (round > 0 && !mbar_wait(empty0 + 8 * s, (round - 1) & 1, args.err, ALTO_ERR_WAIT_EMPTY, bail)) break;
-        const uint32_t sa = base_addr + s * S::kStageBytes, sb = sa + S::kABytes;
+    // ---------------------------------------------------------------- TMA producer (the warp, one lane issuing)
+    // The A operand (database or packing matrix) streams through once per unit; B (limbs) is shared by all units.
+    const uint64_t pol_a = policy_evict_first();
+    const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
+    // record chunk of the unit (scan units lie in one chunk; the pack has one) and its first block's offset in it
+    const int z = EPI == Epi::kScan ? kb0 / args.kb_chunk : 0;
+    int x = (EPI == Epi::kScan ? kb0 - z * args.kb_chunk : kb0) * kBK;
+    int s = 0, phase = 1, issued = 0;  // the first round's stages are free
+    for (int i = 0; i < nkb; ++i, x += kBK) {
+      if (!mbar_wait(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) break;
+      const uint32_t sa = base_addr + (uint32_t)s * S::kStageBytes, sb = sa + S::kABytes;
+      if (elect_one()) {
         mbar_arrive_expect_tx(full0 + 8 * s, S::kStageBytes);
-        if constexpr (EPI == Epi::kScan) {
-          // record chunk z, 128-byte block x inside it
-          const int kb = kb0 + i, z = kb / args.kb_chunk, x = (kb - z * args.kb_chunk) * kBK;
-          tma_load_tile(sa, &map_a, full0 + 8 * s, kb, m_tile, pol_a);
+        tma_load_tile(sa, &map_a, full0 + 8 * s, kb0 + i, m_tile, pol_a);
+        if constexpr (EPI == Epi::kScan)
           tma_load_3d(sb, &map_b, full0 + 8 * s, x, n_tile * BN, z, pol_b);
-        } else {
-          tma_load_tile(sa, &map_a, full0 + 8 * s, kb0 + i, m_tile, pol_a);
-          tma_load_2d(sb, &map_b, full0 + 8 * s, (kb0 + i) * kBK, n_tile * BN, pol_b);
-        }
-        issued = i + 1;
+        else
+          tma_load_2d(sb, &map_b, full0 + 8 * s, x, n_tile * BN, pol_b);
       }
-      if (*bail) {
-        // Drain: the last load issued into each stage must land before the CTA may exit.
-        for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
-          mbar_wait(full0 + 8 * (i % kStages), (i / kStages) & 1, args.err, ALTO_ERR_WAIT_DRAIN, &no_bail);
+      __syncwarp();
+      issued = i + 1;
+      if (++s == kStages) {
+        s = 0;
+        phase ^= 1;
       }
+    }
+    if (*bail) {
+      // Drain: the last load issued into each stage must land before the CTA may exit.
+      for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
+        mbar_wait(full0 + 8 * (i % kStages), (i / kStages) & 1, args.err, ALTO_ERR_WAIT_DRAIN, &no_bail);
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_u8u8_s32(BN);
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % kStages, round = i / kStages;
-        if (!mbar_wait(full0 + 8 * s, round & 1, args.err, ALTO_ERR_WAIT_FULL, bail)) break;
-        tc_fence_after();
-        const uint32_t sa = base_addr + s * S::kStageBytes, sb = sa + S::kABytes;
+    // ---------------------------------------------------------------- MMA issuer (the warp, one lane issuing)
+    constexpr uint32_t idesc = idesc_u8u8_s32(BN);
+    const uint32_t a0 = desc_lo_sw128(base_addr);
+    int s = 0, phase = 0;
+    for (int i = 0; i < nkb; ++i) {
+      if (!mbar_wait(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) break;
+      tc_fence_after();
+      const uint32_t a_lo = a0 + (uint32_t)s * (S::kStageBytes >> 4), b_lo = a_lo + (S::kABytes >> 4);
+      if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < kBK / 32; ++kk)
-          mma_i8(tmem_base, desc_sw128(sa + kk * 32), desc_sw128(sb + kk * 32), idesc, (i | kk) != 0);
+        for (uint32_t kk = 0; kk < kBK / 32; ++kk)
+          mma_i8(tmem_base, desc_of(a_lo + 2 * kk), desc_of(b_lo + 2 * kk), idesc, kk == 0 ? i != 0 : 1u);
         mma_commit(empty0 + 8 * s);
       }
+      __syncwarp();
+      if (++s == kStages) {
+        s = 0;
+        phase ^= 1;
+      }
+    }
+    if (elect_one()) {
       mma_commit(accum);
       if (*bail) mbar_wait(accum, 0, args.err, ALTO_ERR_WAIT_DRAIN, &no_bail);
     }

@@ -20,18 +20,15 @@
 
 namespace alto {
 
-// NSUB = 1: a unit is BN limb columns and TMEM holds two accumulators (the epilogue of one unit overlaps the
-// MMAs of the next).  NSUB = 2: a unit is 2 x BN limb columns in two sub-accumulators that fill TMEM (one buffer),
-// so that every A tile is read once for all of them -- for long scans whose A tiles are too large to be shared
-// between pairs through L2.
-template <int BN, int NSUB = 1>
+// A unit is BN limb columns and TMEM holds two accumulators (the epilogue of one unit overlaps the MMAs of the next).
+template <int BN>
 struct PairShape {
   static constexpr int kABytes = 128 * kBK;                 // this CTA's 128 rows of A
-  static constexpr int kBBytes = NSUB * (BN / 2) * kBK;     // this CTA's BN/2 rows of B for each sub-tile
+  static constexpr int kBBytes = (BN / 2) * kBK;            // this CTA's BN/2 rows of B
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = (196608 / kStageBytes) < 8 ? (196608 / kStageBytes) : 8;
-  static constexpr int kBufs = NSUB == 1 ? 2 : 1;           // accumulator buffers
-  static constexpr int kTmemCols = kBufs * NSUB * BN;
+  static constexpr int kBufs = 2;                           // accumulator buffers
+  static constexpr int kTmemCols = kBufs * BN;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;
   static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "pair kind::i8 MMA needs N in [32, 256], N % 32 == 0");
@@ -42,7 +39,7 @@ struct PairShape {
 
 struct PairArgs {
   int num_m;        // tiles of 256 rows along A
-  int num_n;        // tiles of BN limb columns along B
+  int num_n;        // units along the limb columns
   int num_units;    // num_m * num_n * K chunks
   int kb_total;     // 128-byte blocks of the whole reduction
   int kb_per_unit;  // blocks per K chunk (scan chunks never exceed 256 blocks = 32768 records)
@@ -59,7 +56,6 @@ struct PairArgs {
   int nw = 0;       // limb columns a tile computes: a multiple of 32 <= BN (0: BN).  The B boxes are nw/2 rows
                     // (the tensor map's box), loaded from the tile's origin n nw, and the MMAs run N = nw, so a
                     // batch whose limb columns are not a power of two neither loads nor multiplies padding columns
-                    // (NSUB = 1 only)
 };
 
 // Epilogue of 16 TMEM columns (4 clients x 4 limbs) for one accumulator row of the scan: row = database column.
@@ -73,30 +69,36 @@ __device__ __forceinline__ void scan_epilogue16(const uint32_t *r, int col, bool
   }
 }
 
-// Epilogue of 16 TMEM columns for one accumulator row of the pack: row = (column, plane j); the 4 planes of a column
-// are 4 adjacent lanes of one warp.  Each lane reduces its plane's sum S_j = sum_i G_ij 2^(8i) (< 2^57) once,
-// shifts it into place (< 2^56), and the four planes are summed in 64 bits by two shuffles (< 2^58) before the one
-// final reduction mod Q.
+// Epilogue of 16 TMEM columns (4 clients x 4 limbs) for one accumulator row of the pack: row = (column, plane j); the 4
+// planes of a column are 4 adjacent lanes of one warp.  Each lane's plane sum S_j = sum_i G_ij 2^(8i) (< 2^56) folds once
+// (< 2^38) and shifts into place (< 2^62; the four planes together < 2^63).  The planes are summed while the four clients
+// are dealt out to the four lanes -- two clients to each half, then one to each lane, six shuffles -- so that each lane
+// reduces and stores one client (about 22 instructions a client and row; four lanes reducing all four took about 60).
 __device__ __forceinline__ void pack_epilogue16(const uint32_t *r, int grow, bool row_ok, int c0, int clients,
                                                 int cols, uint32_t *out) {
   const int col = grow >> 2, plane = grow & 3;
+  uint64_t w[4];
 #pragma unroll
   for (int cl = 0; cl < 4; ++cl) {
-    const uint64_t sum = (uint64_t)r[4 * cl] + ((uint64_t)r[4 * cl + 1] << 8) + ((uint64_t)r[4 * cl + 2] << 16) +
-                         ((uint64_t)r[4 * cl + 3] << 24);
-    uint64_t u = mod_q64(sum) << (8 * plane);
-    u += __shfl_xor_sync(0xffffffffu, u, 1);
-    u += __shfl_xor_sync(0xffffffffu, u, 2);
-    const int c = c0 + cl;
-    if (plane == 0 && row_ok && c < clients) out[(size_t)c * cols + col] = (uint32_t)mod_q64(u);
+    const uint64_t lo = (uint64_t)r[4 * cl + 1] * 256u + r[4 * cl], hi = (uint64_t)r[4 * cl + 3] * 256u + r[4 * cl + 2];
+    const uint64_t s = lo + (hi << 16);
+    w[cl] = ((s >> 32) * 12287ull + (s & 0xffffffffull)) << (8 * plane);
   }
+  const bool b1 = plane & 2, b0 = plane & 1;
+  uint64_t k0 = b1 ? w[2] : w[0], k1 = b1 ? w[3] : w[1];
+  k0 += __shfl_xor_sync(0xffffffffu, b1 ? w[0] : w[2], 2);
+  k1 += __shfl_xor_sync(0xffffffffu, b1 ? w[1] : w[3], 2);
+  uint64_t u = b0 ? k1 : k0;
+  u += __shfl_xor_sync(0xffffffffu, b0 ? k0 : k1, 1);
+  const int c = c0 + plane;
+  if (row_ok && c < clients) out[(size_t)c * cols + col] = (uint32_t)mod_q64(u);
 }
 
-template <int BN, Epi EPI, int NSUB = 1>
+template <int BN, Epi EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     limb_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           PairArgs args) {
-  using S = PairShape<BN, NSUB>;
+  using S = PairShape<BN>;
   constexpr int kBufs = S::kBufs;
   constexpr int kStages = S::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -109,8 +111,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   volatile int *bail = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // the tile width: a multiple of 32 in [32, BN] (the host checks), BN with NSUB = 2
-  const int nw = (NSUB == 1 && args.nw >= 32 && args.nw <= BN && args.nw % 32 == 0) ? args.nw : BN;
+  // the tile width: a multiple of 32 in [32, BN] (the host checks)
+  const int nw = (args.nw >= 32 && args.nw <= BN && args.nw % 32 == 0) ? args.nw : BN;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -142,7 +144,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   cluster_sync_all();  // barrier initialisation visible to the peer before any of its loads signal the leader
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  volatile int no_bail = 0;
 
   auto unit_coords = [&](int u, int &m, int &n, int &kb0, int &nkb) {
     n = u % args.num_n;
@@ -153,83 +154,84 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   };
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      // both CTAs' A tiles and B boxes of this stage: the B box is nw/2 rows (the host makes the map with that box)
-      const uint32_t stage_tx = 2u * (uint32_t)(S::kABytes + NSUB * (nw / 2) * kBK);
-      const uint64_t pol_a = policy_evict_first();
-      const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
-      const uint32_t full_leader0 = map_to_rank(full0, 0);
-      int g = 0;
-      bool stop = false;
-      for (int u = pair; u < args.num_units && !stop; u += pairs) {
-        int m, n, kb0, nkb;
-        unit_coords(u, m, n, kb0, nkb);
-        for (int i = 0; i < nkb; ++i, ++g) {
-          const int s = g % kStages, round = g / kStages;
-          if (round > 0 && !mbar_wait(empty0 + 8 * s, (round - 1) & 1, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
-            stop = true;
-            break;
-          }
-          const uint32_t sa = base_addr + s * S::kStageBytes, sb = sa + S::kABytes;
+    // ------------------------------------------------------------ TMA producer (both CTAs; the warp, one lane issuing)
+    // both CTAs' A tiles and B boxes of this stage: the B box is nw/2 rows (the host makes the map with that box)
+    const uint32_t stage_tx = 2u * (uint32_t)(S::kABytes + (nw / 2) * kBK);
+    const uint64_t pol_a = policy_evict_first();
+    const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
+    const uint32_t full_leader0 = map_to_rank(full0, 0);
+    int s = 0, phase = 1;  // the first round's stages are free
+    bool stop = false;
+    for (int u = pair; u < args.num_units && !stop; u += pairs) {
+      int m, n, kb0, nkb;
+      unit_coords(u, m, n, kb0, nkb);
+      const int mt = 2 * m + (int)rank, y = n * nw + (int)rank * (nw / 2);
+      // record chunk of the unit's first block and that block's offset in it (a unit lies in one chunk; the pack has one)
+      const int z = EPI == Epi::kScan ? kb0 / args.kb_chunk : 0;
+      int x = (kb0 - z * args.kb_chunk) * kBK;
+      if (EPI == Epi::kPack) x = kb0 * kBK;
+      for (int i = 0; i < nkb; ++i, x += kBK) {
+        if (!mbar_wait(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
+          stop = true;
+          break;
+        }
+        const uint32_t sa = base_addr + (uint32_t)s * S::kStageBytes, bar = full_leader0 + 8 * s;
+        if (elect_one()) {
           if (leader) mbar_arrive_expect_tx(full0 + 8 * s, stage_tx);
-          if constexpr (EPI == Epi::kScan) {
-            const int kb = kb0 + i, z = kb / args.kb_chunk, x = (kb - z * args.kb_chunk) * kBK;
-            tma_load_tile_pair(sa, &map_a, full_leader0 + 8 * s, kb, 2 * m + (int)rank, pol_a);
-#pragma unroll
-            for (int t = 0; t < NSUB; ++t)
-              tma_load_3d_pair(sb + t * (BN / 2) * kBK, &map_b, full_leader0 + 8 * s, x,
-                               (n * NSUB + t) * nw + (int)rank * (nw / 2), z, pol_b);
-          } else {
-            const int x = (kb0 + i) * kBK;
-            tma_load_tile_pair(sa, &map_a, full_leader0 + 8 * s, kb0 + i, 2 * m + (int)rank, pol_a);
-#pragma unroll
-            for (int t = 0; t < NSUB; ++t)
-              tma_load_2d_pair(sb + t * (BN / 2) * kBK, &map_b, full_leader0 + 8 * s, x,
-                               (n * NSUB + t) * nw + (int)rank * (nw / 2), pol_b);
-          }
+          tma_load_tile_pair(sa, &map_a, bar, kb0 + i, mt, pol_a);
+          if constexpr (EPI == Epi::kScan)
+            tma_load_3d_pair(sa + S::kABytes, &map_b, bar, x, y, z, pol_b);
+          else
+            tma_load_2d_pair(sa + S::kABytes, &map_b, bar, x, y, pol_b);
+        }
+        __syncwarp();
+        if (++s == kStages) {
+          s = 0;
+          phase ^= 1;
         }
       }
-      if (stop) {
-        // loads already issued land within microseconds; give them a bounded while before the CTA may exit
-        const uint64_t t0 = globaltimer();
-        while (globaltimer() - t0 < 200000ull) {
-        }
+    }
+    if (stop) {
+      // loads already issued land within microseconds; give them a bounded while before the CTA may exit
+      const uint64_t t0 = globaltimer();
+      while (globaltimer() - t0 < 200000ull) {
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    if (leader) {  // the whole warp, one lane of it issuing
       const uint32_t idesc = idesc_pair_u8u8_s32((uint32_t)nw);
-      int g = 0, it = 0;
+      const uint32_t a0 = desc_lo_sw128(base_addr);
+      int s = 0, phase = 0, it = 0;
       bool stop = false;
       for (int u = pair; u < args.num_units && !stop; u += pairs, ++it) {
         int m, n, kb0, nkb;
         unit_coords(u, m, n, kb0, nkb);
         const int ab = it % kBufs, use = it / kBufs;
         if (use > 0 && !mbar_wait(acce0 + 8 * ab, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(ab * NSUB * BN);
-        for (int i = 0; i < nkb; ++i, ++g) {
-          const int s = g % kStages, round = g / kStages;
-          if (!mbar_wait(full0 + 8 * s, round & 1, args.err, ALTO_ERR_WAIT_FULL, bail)) {
+        const uint32_t d_tmem = tmem_base + (uint32_t)(ab * BN);
+        for (int i = 0; i < nkb; ++i) {
+          if (!mbar_wait(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) {
             stop = true;
             break;
           }
           tc_fence_after();
-          const uint32_t sa = base_addr + s * S::kStageBytes, sb = sa + S::kABytes;
-#pragma unroll
-          for (int t = 0; t < NSUB; ++t)
-#pragma unroll
-            for (int kk = 0; kk < kBK / 32; ++kk)
-              mma_i8_pair(d_tmem + t * BN, desc_sw128(sa + kk * 32), desc_sw128(sb + t * (BN / 2) * kBK + kk * 32),
-                          idesc, (i | kk) != 0);
-          mma_commit_pair(empty0 + 8 * s);
+          const uint32_t a_lo = a0 + (uint32_t)s * (S::kStageBytes >> 4);
+          if (elect_one()) {
+            mma_block_pair(d_tmem, a_lo, a_lo + (S::kABytes >> 4), idesc, i != 0);
+            mma_commit_pair(empty0 + 8 * s);
+          }
+          __syncwarp();
+          if (++s == kStages) {
+            s = 0;
+            phase ^= 1;
+          }
         }
-        mma_commit_pair(accf0 + 8 * ab);
+        if (elect_one()) mma_commit_pair(accf0 + 8 * ab);
+        __syncwarp();
       }
-      if (*bail) {
+      if (*bail && elect_one()) {
         // every MMA issued so far completes before this CTA (and its TMEM and shared memory) may go away
         mma_commit_pair(accf0);
         const uint64_t t0 = globaltimer();
@@ -250,18 +252,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       const int ab = it % kBufs, use = it / kBufs;
       if (!mbar_wait(accf0 + 8 * ab, use & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) break;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + (uint32_t)(ab * NSUB * BN) + ((uint32_t)(q * 32) << 16);
+      const uint32_t taddr = tmem_base + (uint32_t)(ab * BN) + ((uint32_t)(q * 32) << 16);
       const int grow = m * 256 + (int)rank * 128 + row;
       const bool row_ok = grow < args.rows_a;
       // 32 columns per TMEM load (one wait per 8 clients instead of per 4)
 #pragma unroll 1
-      for (int ch = 0; ch < NSUB * nw / 32; ++ch) {
+      for (int ch = 0; ch < nw / 32; ++ch) {
         uint32_t r[32];
         tmem_ld32(taddr + ch * 32, r);
         tmem_wait_ld();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int c0 = n * NSUB * (nw / 4) + ch * 8 + h * 4;
+          const int c0 = n * (nw / 4) + ch * 8 + h * 4;
           if constexpr (EPI == Epi::kScan)
             scan_epilogue16(r + 16 * h, grow, row_ok, c0, args.clients, args.cols, args.out);
           else
@@ -281,7 +283,225 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, S::kTmemCols);
   }
-  (void)no_bail;
+}
+
+// ------------------------------------------------------------------------------------ wide units
+// Units of 2 x nw limb columns in two sub-accumulators of TMEM (nw a multiple of 32, at most 256), for batches of more
+// than 256 limb columns: each A tile is loaded once for both, 48 KB of operands per 1024 MMA cycles at nw = 256 against
+// 64 in units of 256 columns (L2 delivers about 68 bytes a clock and SM to tiled loads, measured alone).
+// The sub-accumulators leave no room for a second pair, so the epilogue is quick instead: sixteen warps take a whole
+// sub-accumulator into registers (64 columns a warp) and release it before they compute.  Sub 0 is read out under the
+// MMAs of a unit's last block into sub 1, sub 1 under those of the next unit's first block into sub 0.
+constexpr int kWideThreads = 576;  // warp 0 TMA, warp 1 MMA + TMEM owner, warps 2..17 epilogue (four per lane quarter)
+constexpr int kWideRing = 196608;  // bytes of shared memory for the stages: leaves room for a tail CTA beside them
+constexpr int kWideMaxStages = 8;
+constexpr int kWideSmem = kWideRing + 512 + 1024;
+inline int wide_stage_bytes(int nw) { return 128 * kBK + nw * kBK; }
+inline int wide_stages(int nw) {
+  return kWideRing / wide_stage_bytes(nw) < kWideMaxStages ? kWideRing / wide_stage_bytes(nw) : kWideMaxStages;
+}
+
+template <Epi EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
+    limb_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                          PairArgs args, int stages) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  const uint32_t base_addr = (raw_addr + 1023u) & ~1023u;
+  uint8_t *smem = smem_raw + (base_addr - raw_addr);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kWideRing);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kWideMaxStages + 4);
+  volatile int *bail = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nw = args.nw, half = nw / 2;
+  const uint32_t stage_bytes = (uint32_t)(128 * kBK + nw * kBK);
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kWideMaxStages;
+  const uint32_t accf0 = empty0 + 8 * kWideMaxStages, acce0 = accf0 + 16;  // per sub-accumulator
+
+  if (tid == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(accf0 + 8 * t, 1);
+      mbar_init(acce0 + 8 * t, 32);  // 16 epilogue warps x 2 CTAs
+    }
+    *bail = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&map_a);
+    tma_prefetch_desc(&map_b);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(tmem_slot), 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // barrier initialisation visible to the peer before any of its loads signal the leader
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  auto unit_coords = [&](int u, int &m, int &n, int &kb0, int &nkb) {
+    n = u % args.num_n;
+    m = args.m_begin + (u / args.num_n) % args.num_m;
+    const int kc = u / (args.num_n * args.num_m);
+    kb0 = args.kb_begin + kc * args.kb_per_unit;
+    nkb = min(kb0 + args.kb_per_unit, args.kb_total) - kb0;
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer (both CTAs; the warp, one lane issuing)
+    const uint64_t pol_a = policy_evict_first();
+    const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
+    const uint32_t full_leader0 = map_to_rank(full0, 0);
+    int s = 0, phase = 1;  // the first round's stages are free
+    bool stop = false;
+    for (int u = pair; u < args.num_units && !stop; u += pairs) {
+      int m, n, kb0, nkb;
+      unit_coords(u, m, n, kb0, nkb);
+      const int mt = 2 * m + (int)rank;
+      const int y = n * 2 * nw + (int)rank * half;  // this CTA's first row of sub 0; sub 1 is nw further
+      const int z = EPI == Epi::kScan ? kb0 / args.kb_chunk : 0;  // a unit lies in one record chunk; the pack has one
+      int x = (kb0 - z * args.kb_chunk) * kBK;
+      if (EPI == Epi::kPack) x = kb0 * kBK;
+      for (int i = 0; i < nkb; ++i, x += kBK) {
+        if (!mbar_wait(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
+          stop = true;
+          break;
+        }
+        const uint32_t sa = base_addr + (uint32_t)s * stage_bytes, sb = sa + 128 * kBK, bar = full_leader0 + 8 * s;
+        if (elect_one()) {
+          if (leader) mbar_arrive_expect_tx(full0 + 8 * s, 2 * stage_bytes);
+          tma_load_tile_pair(sa, &map_a, bar, kb0 + i, mt, pol_a);
+          if constexpr (EPI == Epi::kScan) {
+            tma_load_3d_pair(sb, &map_b, bar, x, y, z, pol_b);
+            tma_load_3d_pair(sb + half * kBK, &map_b, bar, x, y + nw, z, pol_b);
+          } else {
+            tma_load_2d_pair(sb, &map_b, bar, x, y, pol_b);
+            tma_load_2d_pair(sb + half * kBK, &map_b, bar, x, y + nw, pol_b);
+          }
+        }
+        __syncwarp();
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    if (stop) {
+      // loads already issued land within microseconds; give them a bounded while before the CTA may exit
+      const uint64_t t0 = globaltimer();
+      while (globaltimer() - t0 < 200000ull) {
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer (leader CTA only)
+    if (leader) {  // the whole warp, one lane of it issuing
+      const uint32_t idesc = idesc_pair_u8u8_s32((uint32_t)nw);
+      const uint32_t a0 = desc_lo_sw128(base_addr), step = stage_bytes >> 4, b_off = 128 * kBK >> 4,
+                     sub = (uint32_t)(half * kBK) >> 4;
+      int s = 0, phase = 0, use = 0;
+      bool stop = false;
+      for (int u = pair; u < args.num_units && !stop; u += pairs, ++use) {
+        int m, n, kb0, nkb;
+        unit_coords(u, m, n, kb0, nkb);
+        for (int i = 0; i < nkb; ++i) {
+          if (i == 0 && use > 0 && !mbar_wait(acce0, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) stop = true;
+          if (stop || !mbar_wait(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) {
+            stop = true;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a_lo = a0 + (uint32_t)s * step;
+          if (elect_one()) {
+            mma_block_pair(tmem_base, a_lo, a_lo + b_off, idesc, i != 0);
+            if (i + 1 == nkb) mma_commit_pair(accf0);
+          }
+          __syncwarp();
+          if (i == 0 && use > 0) {
+            if (!mbar_wait(acce0 + 8, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) {
+              stop = true;
+              break;
+            }
+            tc_fence_after();
+          }
+          if (elect_one()) {
+            mma_block_pair(tmem_base + 256, a_lo, a_lo + b_off + sub, idesc, i != 0);
+            mma_commit_pair(empty0 + 8 * s);
+            if (i + 1 == nkb) mma_commit_pair(accf0 + 8);
+          }
+          __syncwarp();
+          if (++s == stages) {
+            s = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (*bail && elect_one()) {
+        // every MMA issued so far completes before this CTA (and its TMEM and shared memory) may go away
+        mma_commit_pair(accf0);
+        const uint64_t t0 = globaltimer();
+        while (globaltimer() - t0 < 200000ull) {
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ epilogue (warps 2..17 of both CTAs)
+    const int q = warp & 3, part = (warp - 2) >> 2;  // lane quarter; chunks part and part + 4 of 32 columns
+    const int row = q * 32 + lane, chunks = nw / 32;
+    const uint32_t acce_leader0 = map_to_rank(acce0, 0);
+    int use = 0;
+    bool stop = false;
+    for (int u = pair; u < args.num_units && !stop; u += pairs, ++use) {
+      int m, n, kb0, nkb;
+      unit_coords(u, m, n, kb0, nkb);
+      const int grow = m * 256 + (int)rank * 128 + row;
+      const bool row_ok = grow < args.rows_a;
+      for (int t = 0; t < 2; ++t) {
+        if (!mbar_wait(accf0 + 8 * t, use & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) {
+          stop = true;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + (uint32_t)t * 256 + ((uint32_t)(q * 32) << 16);
+        uint32_t r[2][32];
+        if (part < chunks) tmem_ld32(taddr + part * 32, r[0]);
+        if (part + 4 < chunks) tmem_ld32(taddr + (part + 4) * 32, r[1]);
+        tmem_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acce_leader0 + 8 * t);
+        const int ct = (n * 2 + t) * (nw / 4);  // first client of the sub-accumulator
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int ch = part + (h >> 1) * 4, c0 = ct + ch * 8 + (h & 1) * 4;
+          if (ch >= chunks) break;
+          const uint32_t *v = r[h >> 1] + 16 * (h & 1);
+          if constexpr (EPI == Epi::kScan)
+            scan_epilogue16(v, grow, row_ok, c0, args.clients, args.cols, args.out);
+          else
+            pack_epilogue16(v, grow, row_ok, c0, args.clients, args.cols, args.out);
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the peer's last arrivals and TMEM reads are done before either CTA frees anything
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
 }
 
 }  // namespace alto
