@@ -985,7 +985,7 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
   // 1 GiB: 376 -> 336 us a call (6.4 TB/s of database and packing matrix); alto_answer 404 -> 358, 251 -> 221 at 64 MiB.
   const bool grouped = e->overlap && slots * e->resp_len >= kGroupedRespBytes;
   const Groups groups = column_groups(e, p, group_weights(grouped ? e->groups : 1, false));
-  const bool scan_on_side = e->overlap && !p.pair && groups.count == 1;
+  const bool scan_on_side = e->overlap && groups.count == 1;
   const int bp = (int)round_up(slots, 4);
   int launches = 0;
   // timing marks (main batch only): 0 begin | validate (one stream only) | 1 | y split | 2 | pack | 3 | (wait for
@@ -1284,7 +1284,7 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
   cudaStream_t vs = e->overlap ? bt->side : st;
   // A small batch's scan follows its query split on the side stream, so validation waits for the z keys on the copy
   // stream instead.
-  const bool scan_on_side = e->overlap && !p.pair && !piped && groups.count == 1;
+  const bool scan_on_side = e->overlap && !piped && groups.count == 1;
   cudaStream_t zs = scan_on_side ? sc : vs;
   if (!piped) {
     ALTO_H(cudaStreamWaitEvent(vs, e->ev_queries, 0));
