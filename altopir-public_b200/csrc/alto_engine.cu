@@ -216,6 +216,10 @@ constexpr size_t kPipedQueryBytes = size_t(32) << 20;
 // of 32 KB records)
 constexpr size_t kGroupedRespBytes = size_t(2) << 20;
 
+// alto_answer uploads frames of at most this many bytes in all at once, as whole frames (10 us of link time): one frame
+// over 64 MiB 222 -> 206 us a call, over 1 GiB 362 -> 350, over 2,048 records x 2 KB 86 -> 60
+constexpr size_t kWholeFrameBytes = size_t(1) << 19;
+
 // ------------------------------------------------------------------------------------------- engine
 // The device resources of one batch in flight: its stream, per-batch scratch (grown on demand) and error word.
 // An engine answers through its `main` batch; a serving loop keeps several so that batches overlap on the device.
@@ -225,7 +229,9 @@ struct Batch {
   uint8_t *d_req = nullptr, *d_qlimb = nullptr, *d_ylimb = nullptr, *d_resp = nullptr;
   int *d_status = nullptr;
   uint32_t *d_acc = nullptr, *d_beta = nullptr;
-  int *h_status = nullptr;
+  int *h_status = nullptr, *hd_status = nullptr;  // pinned statuses that validation stores into, and their device address
+  // the error word: pinned host memory that the kernels store into (d_err is its device address), so that no copy
+  // brings it back
   uint32_t *d_err = nullptr, *h_err = nullptr;
   bool timing = false;  // record per-kernel timing marks into the engine's ring (main batch only)
   // Side stream of the overlapped schedule: the query limb split beside the pack, and the tail of each column group
@@ -403,7 +409,7 @@ void free_scratch(Batch *b) {
   b->d_req = b->d_qlimb = b->d_ylimb = b->d_resp = nullptr;
   b->d_status = nullptr;
   b->d_acc = b->d_beta = nullptr;
-  b->h_status = nullptr;
+  b->h_status = b->hd_status = nullptr;
   b->cap = 0;
 }
 
@@ -419,9 +425,9 @@ bool init_batch(Batch *b, bool timing) {
   for (cudaEvent_t *ev : {&b->ev_fork, &b->ev_qready, &b->ev_join})
     ALTO_CK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
   for (cudaEvent_t &ev : b->ev_scan) ALTO_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  ALTO_CK(cudaMalloc(&b->d_err, sizeof(uint32_t)));
-  ALTO_CK(cudaMemset(b->d_err, 0, sizeof(uint32_t)));
-  ALTO_CK(cudaHostAlloc(&b->h_err, sizeof(uint32_t), cudaHostAllocDefault));
+  ALTO_CK(cudaHostAlloc(&b->h_err, sizeof(uint32_t), cudaHostAllocMapped));
+  *b->h_err = 0;
+  ALTO_CK(cudaHostGetDevicePointer(reinterpret_cast<void **>(&b->d_err), b->h_err, 0));
   b->timing = timing;
   return true;
 }
@@ -432,7 +438,6 @@ void destroy_batch(Batch *b) {
   free_scratch(b);
   cudaFree(b->d_gather);
   b->d_gather = nullptr;
-  cudaFree(b->d_err);
   cudaFreeHost(b->h_err);
   for (cudaEvent_t ev : {b->ev_fork, b->ev_qready, b->ev_join})
     if (ev) cudaEventDestroy(ev);
@@ -491,7 +496,8 @@ bool ensure_capacity(const Engine *e, Batch *b, size_t slots) {
   ALTO_CK(cudaMalloc(&b->d_status, cap * sizeof(int)));
   ALTO_CK(cudaMalloc(&b->d_acc, cap * e->cols * sizeof(uint32_t)));
   ALTO_CK(cudaMalloc(&b->d_beta, cap * e->cols * sizeof(uint32_t)));
-  ALTO_CK(cudaHostAlloc(&b->h_status, cap * sizeof(int), cudaHostAllocDefault));
+  ALTO_CK(cudaHostAlloc(&b->h_status, cap * sizeof(int), cudaHostAllocMapped));
+  ALTO_CK(cudaHostGetDevicePointer(reinterpret_cast<void **>(&b->hd_status), b->h_status, 0));
   b->cap = cap;
   return true;
 }
@@ -926,6 +932,32 @@ bool enqueue_query_split(const Engine *e, const Batch *bt, const uint8_t *d_slot
   return true;
 }
 
+// Splits, validation and zeroing for `slots` staged frames in one launch on stream st (prep_kernel).
+bool enqueue_prep(const Engine *e, const Batch *bt, const uint8_t *d_slots, size_t slot_stride, size_t slots,
+                  bool host_status, cudaStream_t st) {
+  alto::PrepArgs a;
+  a.req = d_slots;
+  a.stride = slot_stride;
+  a.lead = kSlotLead;
+  a.count = e->count;
+  a.rows = e->rows;
+  a.chunk = e->chunk;
+  a.slots = (int)slots;
+  a.padded = (int)round_up(slots, 4);
+  a.ylimb = bt->d_ylimb;
+  a.qlimb = bt->d_qlimb;
+  a.status = bt->d_status;
+  a.host_status = host_status ? bt->hd_status : nullptr;
+  a.acc = bt->d_acc;
+  a.acc_words = slots * e->cols;
+  a.y_blocks = (unsigned)(((e->count / 16) * a.padded + 255) / 256);
+  a.q_blocks = (unsigned)(((e->rows / 16) * a.padded + 255) / 256);
+  const unsigned zero_blocks = (unsigned)((a.acc_words + 4095) / 4096);
+  alto::prep_kernel<<<a.y_blocks + a.q_blocks + (unsigned)slots + zero_blocks, 256, 0, st>>>(a);
+  ALTO_CK(cudaGetLastError());
+  return true;
+}
+
 // Scan and tail in column groups: the tail of every group but the last runs on the side stream beside the scan of the
 // next group (the tail is integer-ALU work, the scan tensor work; the side stream's lower priority lets the scan's
 // CTAs be placed first); `done[g]`, when given, is recorded after the tail of group g.
@@ -976,7 +1008,8 @@ bool enqueue_scan_tails(Engine *e, Batch *bt, const Plan &p, const CUtensorMap &
 // tails of all column groups but the last beside the scan (enqueue_scan_tails); the side stream forks from and joins
 // back into the batch's stream, so the batch is complete when its stream passes it.
 bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t slot_stride, size_t slots,
-                          uint8_t *resp, size_t resp_stride, bool host_status, bool with_marks) {
+                          uint8_t *resp, size_t resp_stride, bool host_status, bool with_marks,
+                          cudaEvent_t pack_done = nullptr) {
   cudaStream_t st = bt->st;
   const Plan p = make_plan(e, slots);
   // A batch of few response bytes scans in one launch, as in answer_host.  With the single-CTA kernels (HBM-bound, two
@@ -1000,29 +1033,37 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
   }
   auto mark = [&](int i) { return mk ? cudaEventRecord(mk[i], st) : cudaSuccess; };
   ALTO_CK(mark(0));
-  // validation (its statuses are needed by the tails only) and the query limb split: on the side stream when the
-  // schedule has two, joined before the scan
-  cudaStream_t vs = st;
-  if (e->overlap) {
-    vs = bt->side;
+  if (scan_on_side) {
+    // everything before the GEMMs in one launch, then the pack here and the scan on the side stream
+    if (!enqueue_prep(e, bt, d_slots, slot_stride, slots, host_status, st)) return false;
+    ++launches;
     ALTO_CK(cudaEventRecord(bt->ev_fork, st));
-    ALTO_CK(cudaStreamWaitEvent(vs, bt->ev_fork, 0));
+    ALTO_CK(cudaStreamWaitEvent(bt->side, bt->ev_fork, 0));
+    ALTO_CK(mark(1));
+  } else {
+    // validation (its statuses are needed by the tails only) and the query limb split: on the side stream when the
+    // schedule has two, joined before the scan
+    cudaStream_t vs = st;
+    if (e->overlap) {
+      vs = bt->side;
+      ALTO_CK(cudaEventRecord(bt->ev_fork, st));
+      ALTO_CK(cudaStreamWaitEvent(vs, bt->ev_fork, 0));
+    }
+    alto::validate_kernel<<<(unsigned)slots, 256, 0, vs>>>(d_slots, slot_stride, kSlotLead, e->count, bt->d_status,
+                                                           host_status ? bt->hd_status : nullptr);
+    ++launches;
+    ALTO_CK(cudaGetLastError());
+    if (e->overlap) {
+      if (!enqueue_query_split(e, bt, d_slots, slot_stride, slots, vs)) return false;
+      launches += 1;
+      ALTO_CK(cudaEventRecord(bt->ev_qready, vs));
+    }
+    ALTO_CK(mark(1));
   }
-  alto::validate_kernel<<<(unsigned)slots, 256, 0, vs>>>(d_slots, slot_stride, kSlotLead, e->count, e->rows,
-                                                         bt->d_status);
-  ++launches;
-  ALTO_CK(cudaGetLastError());
-  if (host_status) ALTO_CK(cudaMemcpyAsync(bt->h_status, bt->d_status, slots * sizeof(int), cudaMemcpyDeviceToHost, vs));
-  if (e->overlap) {
-    if (!enqueue_query_split(e, bt, d_slots, slot_stride, slots, vs)) return false;
-    launches += 1;
-    ALTO_CK(cudaEventRecord(bt->ev_qready, vs));
-  }
-  ALTO_CK(mark(1));
 
   CUtensorMap map_q, map_y;
   if (!make_limb_maps(e, p, bt->d_qlimb, bt->d_ylimb, bp, &map_q, &map_y)) return false;
-  {
+  if (!scan_on_side) {
     const size_t work = (e->count / 16) * (size_t)bp;
     alto::limb_split_kernel<<<(unsigned)((work + 255) / 256), 256, 0, st>>>(
         d_slots, slot_stride, kSlotLead + 9, (int)slots, bp, e->count, e->count, bt->d_ylimb);
@@ -1033,8 +1074,9 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
   if (!launch_pack(e, p, map_y, bt->d_beta, slots, st, bt->d_err)) return false;
   ++launches;
   ALTO_CK(mark(3));
+  if (pack_done) ALTO_CK(cudaEventRecord(pack_done, st));
   if (scan_on_side) {
-    // the scan follows the query split on the side stream
+    // the scan follows the preparation on the side stream
   } else if (e->overlap) {
     ALTO_CK(cudaStreamWaitEvent(st, bt->ev_qready, 0));
   } else {
@@ -1118,13 +1160,10 @@ bool copy_runs(size_t items, size_t width, SrcAt src_at, DstAt dst_at, cudaMemcp
 
 // Waits for the engine's stream, folds pending timing marks into the totals and checks (then clears) the device
 // error word.
-// After a batch's stream has passed a copy of its error word into the pinned mirror: false (and the word reset)
-// when a kernel wait timed out.
+// After a batch's stream has been waited for: false (and the word reset) when a kernel wait timed out.
 bool check_batch_error(Batch *b) {
   const uint32_t err = *b->h_err;
   if (err) {
-    ALTO_CK(cudaMemsetAsync(b->d_err, 0, sizeof(uint32_t), b->st));
-    ALTO_CK(cudaStreamSynchronize(b->st));
     *b->h_err = 0;
     char buf[96];
     snprintf(buf, sizeof buf, "a kernel wait timed out (device error word 0x%x)", err);
@@ -1142,11 +1181,9 @@ bool sync_engine(Engine *e) {
   bool ok = true;
   for (int k = e->lanes_made - 1; k >= 1; --k) {
     Batch *b = &e->lane[k - 1];
-    ALTO_CK(cudaMemcpyAsync(b->h_err, b->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, b->st));
     ALTO_CK(cudaStreamSynchronize(b->st));
     ok = check_batch_error(b) && ok;
   }
-  ALTO_CK(cudaMemcpyAsync(e->main.h_err, e->main.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->main.st));
   ALTO_CK(cudaStreamSynchronize(e->main.st));
   return check_error_word(e) && ok;
 }
@@ -1230,6 +1267,42 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
       return -4;                       \
     }                                  \
   } while (0)
+  if (e->overlap && groups.count == 1 && nc * e->want <= kWholeFrameBytes) {
+    // A few small frames upload whole and run as a device batch: the overlap of their uploads with the pack is worth
+    // less than the dozen calls that it takes.
+    if (stage_ms) ALTO_H(cudaEventRecord(e->ev_begin, st));
+    if (!copy_runs(
+            nc, e->want, [&](size_t i) { return (const void *)req[cand[i]]; },
+            [&](size_t i) { return (void *)(bt->d_req + i * e->slot_stride + kSlotLead); }, cudaMemcpyHostToDevice, st))
+      return -4;
+    if (stage_ms) ALTO_H(cudaEventRecord(e->ev_keys, st));
+    if (!enqueue_batch_direct(e, bt, bt->d_req, e->slot_stride, nc, bt->d_resp, e->resp_len, true, false,
+                              stage_ms ? e->ev_pack : nullptr))
+      return -4;
+    if (stage_ms) ALTO_H(cudaEventRecord(e->ev_group[0], st));
+    ALTO_H(cudaEventSynchronize(bt->ev_fork));  // the statuses are in
+    std::vector<size_t> ok;
+    for (size_t i = 0; i < nc; ++i) {
+      status[cand[i]] = bt->h_status[i];
+      if (bt->h_status[i] == 0) ok.push_back(i);
+    }
+    if (!copy_runs(
+            ok.size(), e->resp_len, [&](size_t k) { return (const void *)(bt->d_resp + ok[k] * e->resp_len); },
+            [&](size_t k) { return (void *)out[cand[ok[k]]]; }, cudaMemcpyDeviceToHost, st))
+      return -4;
+    if (stage_ms) ALTO_H(cudaEventRecord(e->ev_end, st));
+    ALTO_H(cudaStreamSynchronize(st));
+    if (!check_error_word(e)) return -4;
+    if (stage_ms) {
+      float t[4];
+      ALTO_H(cudaEventElapsedTime(&t[0], e->ev_begin, e->ev_keys));
+      ALTO_H(cudaEventElapsedTime(&t[1], e->ev_pack, e->ev_group[0]));
+      ALTO_H(cudaEventElapsedTime(&t[2], e->ev_keys, e->ev_pack));
+      ALTO_H(cudaEventElapsedTime(&t[3], e->ev_group[0], e->ev_end));
+      std::copy(t, t + 4, stage_ms);
+    }
+    return (int)ok.size();
+  }
   ALTO_H(cudaEventRecord(e->ev_begin, st));
   if (!copy_runs(
           nc, ybytes, [&](size_t i) { return (const void *)req[cand[i]]; },
@@ -1307,11 +1380,10 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
     }
   }
   ALTO_H(cudaStreamWaitEvent(zs, e->ev_zkeys, 0));
-  alto::validate_kernel<<<(unsigned)nc, 256, 0, zs>>>(bt->d_req, e->slot_stride, kSlotLead, e->count, e->rows,
-                                                      bt->d_status);
+  alto::validate_kernel<<<(unsigned)nc, 256, 0, zs>>>(bt->d_req, e->slot_stride, kSlotLead, e->count, bt->d_status,
+                                                      bt->hd_status);
   ALTO_H(cudaGetLastError());
   ++launches;
-  ALTO_H(cudaMemcpyAsync(bt->h_status, bt->d_status, nc * sizeof(int), cudaMemcpyDeviceToHost, zs));
   ALTO_H(cudaEventRecord(e->ev_status, zs));
   // The scan in column groups (with the tails and downloads) covers the last quarter of the chunk groups, which it
   // starts once all query words are in; the chunk groups before it scan all columns as they arrive.  The upload of
@@ -1340,8 +1412,6 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
                           e->ev_group, &launches, nullptr, e->ev_status, groups.count - e->host_inline - 1, kb_last,
                           scan_on_side))
     return -4;
-  // the error word comes back behind the last tail, so the final synchronisation covers it
-  ALTO_H(cudaMemcpyAsync(bt->h_err, bt->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   e->last_launches = launches;
 
   // statuses come back as soon as validation is done; then each group's valid responses download on the copy
@@ -1666,9 +1736,9 @@ int alto_answer_device(void *p, const uint8_t *d_req, size_t req_stride, size_t 
   if (!b) return 0;
   if (!e->tail_ok) return -3;
   if (cudaSetDevice(e->dev) != cudaSuccess || !ensure_capacity(e, &e->main, b)) return -4;
-  if (cudaEventRecord(e->ev_begin, e->main.st) != cudaSuccess) return -4;
+  if (stage_ms && cudaEventRecord(e->ev_begin, e->main.st) != cudaSuccess) return -4;
   if (!enqueue_batch(e, &e->main, d_req, req_stride, b, d_out, out_stride, true)) return -4;
-  if (cudaEventRecord(e->ev_end, e->main.st) != cudaSuccess) return -4;
+  if (stage_ms && cudaEventRecord(e->ev_end, e->main.st) != cudaSuccess) return -4;
   if (!finish(e, stage_ms)) return -4;
   int valid = 0;
   for (size_t c = 0; c < b; ++c) {
@@ -2110,7 +2180,6 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
     step(cudaGetLastError());
     // the engine's tail twiddles: its inverse table psi^-brv / 2, doubled as create_engine stores it
     step(cudaMemcpyAsync(e->d_tw, d_psi_inv, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, 0));
-    step(cudaMemcpyAsync(e->main.h_err, e->main.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, 0));
     step(cudaEventRecord(t1, 0));
     step(cudaEventSynchronize(t1));
   }
@@ -2264,22 +2333,31 @@ bool enqueue_noalloc(Engine *e, uint8_t *scratch, const NoAllocLayout &l, const 
   uint8_t *qlimb = scratch + l.qlimb, *ylimb = scratch + l.ylimb;
   uint32_t *acc = reinterpret_cast<uint32_t *>(scratch + l.acc), *beta = reinterpret_cast<uint32_t *>(scratch + l.beta);
   const unsigned split_threads = 256;
-
-  alto::validate_kernel<<<(unsigned)b, 256, 0, st>>>(d_slots, stride, kSlotLead, e->count, e->rows, status);
-  ALTO_CK(cudaGetLastError());
-  const size_t qwork = (e->rows / 16) * (size_t)bp;
-  alto::limb_split_kernel<<<(unsigned)((qwork + split_threads - 1) / split_threads), split_threads, 0, st>>>(
-      d_slots, stride, kSlotLead + 9 + 8 * e->count, (int)b, bp, e->rows, e->chunk, qlimb);
-  ALTO_CK(cudaGetLastError());
-  ALTO_CK(cudaMemsetAsync(acc, 0, b * e->cols * sizeof(uint32_t), st));  // the scan adds into these sums
+  // the query split and the scan beside the key split and the pack (one stream without the overlapped schedule)
+  cudaStream_t side = e->overlap ? e->main.side : st;
+  if (side != st) {
+    ALTO_CK(cudaEventRecord(e->main.ev_fork, st));
+    ALTO_CK(cudaStreamWaitEvent(side, e->main.ev_fork, 0));
+  }
+  CUtensorMap map_q, map_y;
+  if (!make_limb_maps(e, p, qlimb, ylimb, bp, &map_q, &map_y)) return false;
   const size_t ywork = (e->count / 16) * (size_t)bp;
   alto::limb_split_kernel<<<(unsigned)((ywork + split_threads - 1) / split_threads), split_threads, 0, st>>>(
       d_slots, stride, kSlotLead + 9, (int)b, bp, e->count, e->count, ylimb);
   ALTO_CK(cudaGetLastError());
-  CUtensorMap map_q, map_y;
-  if (!make_limb_maps(e, p, qlimb, ylimb, bp, &map_q, &map_y)) return false;
-  if (!launch_scan(e, p, map_q, acc, b, st, e->main.d_err)) return false;
   if (!launch_pack(e, p, map_y, beta, b, st, e->main.d_err)) return false;
+  const size_t qwork = (e->rows / 16) * (size_t)bp;
+  alto::limb_split_kernel<<<(unsigned)((qwork + split_threads - 1) / split_threads), split_threads, 0, side>>>(
+      d_slots, stride, kSlotLead + 9 + 8 * e->count, (int)b, bp, e->rows, e->chunk, qlimb);
+  ALTO_CK(cudaGetLastError());
+  ALTO_CK(cudaMemsetAsync(acc, 0, b * e->cols * sizeof(uint32_t), side));  // the scan adds into these sums
+  if (!launch_scan(e, p, map_q, acc, b, side, e->main.d_err)) return false;
+  alto::validate_kernel<<<(unsigned)b, 256, 0, st>>>(d_slots, stride, kSlotLead, e->count, status, nullptr);
+  ALTO_CK(cudaGetLastError());
+  if (side != st) {
+    ALTO_CK(cudaEventRecord(e->main.ev_scan[0], side));
+    ALTO_CK(cudaStreamWaitEvent(st, e->main.ev_scan[0], 0));
+  }
   alto::TailArgs t;
   t.acc = acc;
   t.beta = beta;
@@ -2334,20 +2412,11 @@ extern "C" int alto_answer_device_noalloc(void *p, const uint8_t *d_req, size_t 
   uint8_t *scratch = nullptr;
   if (!noalloc_scratch(e->dev, &scratch)) return -4;
   if (!enqueue_noalloc(e, scratch, l, d_req, req_stride, b, d_out, out_stride, d_status)) return -4;
-  // wait and check the engine's device error word (its pinned host mirror already exists)
-  if (cudaMemcpyAsync(e->main.h_err, e->main.d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->main.st) != cudaSuccess ||
-      cudaStreamSynchronize(e->main.st) != cudaSuccess) {
+  if (cudaStreamSynchronize(e->main.st) != cudaSuccess) {
     set_error("allocation-free batch failed", cudaGetLastError());
     return -4;
   }
-  if (*e->main.h_err) {
-    char buf[96];
-    snprintf(buf, sizeof buf, "a kernel wait timed out (device error word 0x%x)", *e->main.h_err);
-    set_error(buf);
-    cudaMemsetAsync(e->main.d_err, 0, sizeof(uint32_t), e->main.st);
-    cudaStreamSynchronize(e->main.st);
-    return -4;
-  }
+  if (!check_batch_error(&e->main)) return -4;
   return 0;
 }
 

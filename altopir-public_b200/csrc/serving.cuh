@@ -209,11 +209,10 @@ bool enqueue_serving(Server *s, ServeSlot &sl, size_t nc) {
   // validation, status download and query limb split beside the pack
   ALTO_CK(cudaEventRecord(bt->ev_fork, st));
   ALTO_CK(cudaStreamWaitEvent(vs, bt->ev_fork, 0));
-  alto::validate_kernel<<<(unsigned)nc, 256, 0, vs>>>(bt->d_req, e->slot_stride, kSlotLead, e->count, e->rows,
-                                                      bt->d_status);
+  alto::validate_kernel<<<(unsigned)nc, 256, 0, vs>>>(bt->d_req, e->slot_stride, kSlotLead, e->count, bt->d_status,
+                                                      bt->hd_status);
   ALTO_CK(cudaGetLastError());
   ++launches;
-  ALTO_CK(cudaMemcpyAsync(bt->h_status, bt->d_status, nc * sizeof(int), cudaMemcpyDeviceToHost, vs));
   ALTO_CK(cudaEventRecord(sl.ev_valid, vs));
   const size_t gsz = (e->nchunks + kQueryGroups - 1) / kQueryGroups;  // chunks per group
   const int qgroups = piped ? (int)((e->nchunks + gsz - 1) / gsz) : 1;
@@ -302,7 +301,6 @@ bool enqueue_serving(Server *s, ServeSlot &sl, size_t nc) {
                           &launches, nullptr, nullptr, 8, kb_last))
     return false;
   ALTO_CK(cudaMemcpyAsync(sl.h_out, bt->d_resp, nc * s->resp_len, cudaMemcpyDeviceToHost, st));
-  ALTO_CK(cudaMemcpyAsync(bt->h_err, bt->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   ALTO_CK(cudaEventRecord(sl.done, st));
   e->last_launches = launches;
   return true;
@@ -518,11 +516,7 @@ void completer_loop(Server *s) {
         cudaEventElapsedTime(&ms[2], sl.ev_pack, sl.done);
         cudaEventElapsedTime(&ms[3], sl.ev0, sl.done);
       }
-      if (*sl.b.h_err) {  // a kernel wait timed out: clear the word for the next batch of this context
-        cudaMemsetAsync(sl.b.d_err, 0, sizeof(uint32_t), sl.b.st);
-        cudaStreamSynchronize(sl.b.st);
-        *sl.b.h_err = 0;
-      }
+      *sl.b.h_err = 0;  // cleared for the next batch of this context
       if (!ok) sl.failed = true;
     }
     // responses out of the context, outside the lock (a ticket's response is read only once it is done)

@@ -10,7 +10,7 @@
 #define ALTO_WAIT_NS 2000000000ull  // 2 s: far above any legitimate wait (a whole batch takes milliseconds)
 #endif
 
-// Error bits written to the device error word.
+// Error codes written to the error word, which is pinned host memory (a plain store; the last one stays).
 enum : uint32_t {
   ALTO_ERR_WAIT_FULL = 1u,    // MMA issuer gave up waiting for a TMA stage
   ALTO_ERR_WAIT_EMPTY = 2u,   // producer gave up waiting for a stage to be released
@@ -84,7 +84,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     if ((it & 63u) == 63u) {
       if (*bail) return false;
       if (globaltimer() - t0 > ALTO_WAIT_NS) {
-        atomicOr(err, code);
+        *reinterpret_cast<volatile uint32_t *>(err) = code;
         *bail = 1;
         return false;
       }
