@@ -216,9 +216,10 @@ constexpr size_t kPipedQueryBytes = size_t(32) << 20;
 // of 32 KB records)
 constexpr size_t kGroupedRespBytes = size_t(2) << 20;
 
-// alto_answer uploads frames of at most this many bytes in all at once, as whole frames (10 us of link time): one frame
-// over 64 MiB 222 -> 206 us a call, over 1 GiB 362 -> 350, over 2,048 records x 2 KB 86 -> 60
-constexpr size_t kWholeFrameBytes = size_t(1) << 19;
+// alto_answer uploads frames of at most this many bytes in all at once, as whole frames (40 us of link time): one frame
+// over 64 MiB 222 -> 206 us a call, over 1 GiB 362 -> 350, over 2,048 records x 2 KB 86 -> 60; ten frames over 4 MiB
+// (0.75 MB) 98 -> 81.  With 8 MB the upload no longer hides: twelve frames over 1 GiB (7 MB) 358 -> 376.
+constexpr size_t kWholeFrameBytes = size_t(1) << 21;
 
 // ------------------------------------------------------------------------------------------- engine
 // The device resources of one batch in flight: its stream, per-batch scratch (grown on demand) and error word.

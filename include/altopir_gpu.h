@@ -76,7 +76,7 @@ size_t alto_response_len(const void *engine);
  *   out[c] (alto_response_len bytes) is written for status 0 only, other output buffers stay untouched.
  * method must be 0 (the reference's AMX code) or 2 (VNNI); both run the same GPU path.  The header and y keys upload
  * first and the pack runs while the z keys and query words upload; the scan and tail then run in column groups
- * whose responses download while the next group computes.  A few small frames (512 KB in all) upload whole instead and
+ * whose responses download while the next group computes.  A few small frames (2 MB in all) upload whole instead and
  * their scan runs beside the pack.  When stage_ms is not NULL it receives device times in
  * ms: [0] header and y-key upload, [1] validation, query split, scans and tails, [2] key split and pack, [3] the
  * last group's download.
