@@ -216,6 +216,8 @@ constexpr size_t kPipedQueryBytes = size_t(32) << 20;
 // of 32 KB records)
 constexpr size_t kGroupedRespBytes = size_t(2) << 20;
 
+// a device batch with more bytes of query words, or of responses, scans in two column groups (device_groups)
+constexpr size_t kHiddenSplitBytes = size_t(32) << 20, kHiddenTailBytes = size_t(32) << 20;
 // alto_answer uploads frames of at most this many bytes in all at once, as whole frames (40 us of link time): one frame
 // over 64 MiB 222 -> 206 us a call, over 1 GiB 362 -> 350, over 2,048 records x 2 KB 86 -> 60; ten frames over 4 MiB
 // (0.75 MB) 98 -> 81.  With 8 MB the upload no longer hides: twelve frames over 1 GiB (7 MB) 358 -> 376.
@@ -305,7 +307,7 @@ struct Engine {
   std::atomic<int> last_launches{0};  // written by whichever thread enqueued the latest batch (a serving loop's too)
   bool use_graphs = false;  // replay captured launch sequences (alto_engine_set_graphs)
   bool overlap = true;      // the two-stream schedule of a batch (ALTO_OVERLAP=0 runs it on one stream)
-  int groups = 2;           // column groups of the scan and tail of a device batch (ALTO_GROUPS: 1, 2, 4 or 8)
+  int groups = 0;           // column groups of the scan and tail of a device batch (ALTO_GROUPS: 1 to 8; 0: device_groups)
   // The column groups of alto_answer, whose downloads overlap the scan, as weights (ALTO_HOST_WEIGHTS, or
   // ALTO_HOST_GROUPS groups with a last one of half the size).  A group's side-stream tail runs once the next group's
   // scan has left the SMs; the tails of the last host_inline groups before the last run on the batch's stream
@@ -1002,6 +1004,18 @@ bool enqueue_scan_tails(Engine *e, Batch *bt, const Plan &p, const CUtensorMap &
   return true;
 }
 
+// Column groups of a device batch.  One, with the preparation in one launch and the scan on the side stream without
+// waiting for the pack (its units fill the SMs as the pack's run out, instead of starting on an idle device), unless the
+// query split is long enough to be worth hiding beside the pack, or the tails enough to be worth hiding beside the scan:
+// then two, the first one's tails beside the second one's scan.  us a call, two groups / one: 1 GiB, one client 376 / 336,
+// 128 clients 856 / 845, four batches of 128 on two lanes 3,345 / 3,310; 8 GiB, 100 clients (105 MB of query words)
+// 3,094 / 3,115.
+int device_groups(const Engine *e, size_t slots) {
+  if (!e->overlap || slots * e->resp_len < kGroupedRespBytes) return 1;
+  if (e->groups) return e->groups;
+  return 4 * slots * e->rows > kHiddenSplitBytes || slots * e->resp_len > kHiddenTailBytes ? 2 : 1;
+}
+
 // Enqueues the answer path for `slots` staged frames on the batch's stream: validate, key limb split, pack GEMM,
 // query limb split, scan GEMM and tail.  Statuses go to d_status (and to the pinned host copy when host_status);
 // responses of valid frames to resp + slot * resp_stride.  With the overlapped schedule validation, the query limb
@@ -1013,12 +1027,7 @@ bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t s
                           cudaEvent_t pack_done = nullptr) {
   cudaStream_t st = bt->st;
   const Plan p = make_plan(e, slots);
-  // A batch of few response bytes scans in one launch, as in answer_host.  With the single-CTA kernels (HBM-bound, two
-  // CTAs an SM) the scan also follows its query split on the side stream without waiting for the pack: its units fill
-  // the SMs as the pack's run out, instead of starting on an idle device after the pack's last one.  One frame over
-  // 1 GiB: 376 -> 336 us a call (6.4 TB/s of database and packing matrix); alto_answer 404 -> 358, 251 -> 221 at 64 MiB.
-  const bool grouped = e->overlap && slots * e->resp_len >= kGroupedRespBytes;
-  const Groups groups = column_groups(e, p, group_weights(grouped ? e->groups : 1, false));
+  const Groups groups = column_groups(e, p, group_weights(device_groups(e, slots), false));
   const bool scan_on_side = e->overlap && groups.count == 1;
   const int bp = (int)round_up(slots, 4);
   int launches = 0;

@@ -296,7 +296,7 @@ bool enqueue_serving(Server *s, ServeSlot &sl, size_t nc) {
     ALTO_CK(cudaStreamWaitEvent(st, sl.ev_sgrp[qgroups - 1], 0));
     kb_last = (int)(r0 / alto::kBK);
   }
-  const Groups groups = column_groups(e, ps, group_weights(e->overlap ? e->groups : 1, false));
+  const Groups groups = column_groups(e, ps, group_weights(!e->overlap ? 1 : e->groups ? e->groups : 2, false));
   if (!enqueue_scan_tails(e, bt, ps, map_q, bt->d_req, e->slot_stride, nc, bt->d_resp, s->resp_len, groups, nullptr,
                           &launches, nullptr, nullptr, 8, kb_last))
     return false;
