@@ -2121,7 +2121,10 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   // n = 2048 with one digit a CTA: the walk with register transforms (ALTO_OFFLINE_WALK8=0 runs the other)
   bool walk8 = n == 2048 && cluster == (int)tg;
   if (const char *v = getenv("ALTO_OFFLINE_WALK8")) walk8 = walk8 && v[0] != '0';
-  const size_t walk8_smem = (3 + 2 * (size_t)cluster) * n * sizeof(uint32_t);
+  const size_t walk8_smem = (alto::kRegWords + (1 + 2 * (size_t)cluster) * n) * sizeof(uint32_t);
+  if (n == 2048)
+    step(cudaFuncSetAttribute(alto::offline_rows8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(alto::kRegWords * sizeof(uint32_t))));
   if (walk8)
     step(cudaFuncSetAttribute(alto::offline_walk8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)walk8_smem));
@@ -2147,7 +2150,8 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
     }
     step(cudaGetLastError());
     if (n == 2048)
-      alto::offline_rows8_kernel<<<(unsigned)std::min<size_t>(cols, 2 * (size_t)sms), 512>>>(d_act, (int)cols, d_psi);
+      alto::offline_rows8_kernel<<<(unsigned)std::min<size_t>(cols, 2 * (size_t)sms), 512,
+                                   alto::kRegWords * sizeof(uint32_t)>>>(d_act, (int)cols, d_psi);
     else
       alto::offline_rows_kernel<<<(unsigned)cols, nt, n * sizeof(uint32_t)>>>(d_act, (int)n, d_psi);
     step(cudaGetLastError());

@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(1024) offline_walk_cluster_kernel(const uint32
 // 512 threads hold 4 values each.  Layout s: index i = (g >> s) << (s + 2) | m << s | (g & (2^s - 1)), so a thread's four
 // values differ in bits s and s + 1.  The inverse transform runs two stages in each of the layouts 0, 2, 4, 6, 8 and the
 // last one (t = 1024) in layout 9; the forward transform the same backwards.  Between layouts the values go through
-// shared memory at swz4(i), free of bank conflicts in every layout.  0 <-> 2 <-> 4 stay inside a warp, 4 <-> 6 inside
+// shared memory, padded against bank conflicts (reg_pad).  0 <-> 2 <-> 4 stay inside a warp, 4 <-> 6 inside
 // two warps and 6 <-> 8 inside eight, so that only 8 <-> 9 needs a barrier of the whole block.  Twiddles are in
 // Montgomery form.
 struct RegTwiddles {
@@ -494,29 +494,22 @@ __device__ __forceinline__ void load_tw(RegTwiddles &t, const uint32_t *__restri
   t.d = to_mont(__ldg(psi + 1));
 }
 
-__device__ __forceinline__ int swz4(int i) { return i ^ (((i >> 5) & 1) << 2) ^ (((i >> 6) & 1) * 0x18); }
 template <int S>
 __device__ __forceinline__ int reg_index(int g, int m) {
   return ((g >> S) << (S + 2)) | (m << S) | (g & ((1 << S) - 1));
 }
+// Every exchange (layouts S and S + 2; 8 and 9 for S = 8) has a buffer of its own, so that a thread only ever overwrites
+// words that it read itself the last time.  Index i lies there at reg_pad(i), padded so that both layouts' accesses are
+// free of bank conflicts; the padding adds, so that the four values of a thread lie at fixed distances from its first.
 template <int S>
-__device__ __forceinline__ void put4(uint32_t *buf, const uint32_t (&x)[4], int g) {
-  if constexpr (S == 0) {
-    *reinterpret_cast<uint4 *>(buf + swz4(4 * g)) = make_uint4(x[0], x[1], x[2], x[3]);
-  } else {
-#pragma unroll
-    for (int m = 0; m < 4; ++m) buf[swz4(reg_index<S>(g, m))] = x[m];
-  }
+__device__ __forceinline__ constexpr int reg_pad(int i) {
+  return S == 0 ? i + 4 * (i >> 5) : S == 2 ? 2304 + i + 20 * (i >> 4) : S == 4 ? 6912 + i + 16 * (i >> 6) : 9472 + (S - 6) * 1024 + i;
 }
-template <int S>
-__device__ __forceinline__ void get4(const uint32_t *buf, uint32_t (&x)[4], int g) {
-  if constexpr (S == 0) {
-    const uint4 u = *reinterpret_cast<const uint4 *>(buf + swz4(4 * g));
-    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
-  } else {
-#pragma unroll
-    for (int m = 0; m < 4; ++m) x[m] = buf[swz4(reg_index<S>(g, m))];
-  }
+constexpr int kRegWords = 13568;  // of the five buffers
+// Layout A's value m in the buffer of exchange S, relative to value 0: bits A and A + 1 of the other index bits are zero.
+template <int S, int A>
+__device__ __forceinline__ constexpr int reg_step(int m) {
+  return reg_pad<S>(m << A) - reg_pad<S>(0);
 }
 __device__ __forceinline__ void sync_warps(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -525,12 +518,25 @@ __device__ __forceinline__ void sync_warps(int id, int threads) {
 template <int A, int B>
 __device__ __forceinline__ void relayout(uint32_t (&x)[4], uint32_t *buf, int g) {
   constexpr int S = A < B ? A : B;
-  put4<A>(buf, x, g);
+  uint32_t *to = buf + reg_pad<S>(reg_index<A>(g, 0));
+  const uint32_t *from = buf + reg_pad<S>(reg_index<B>(g, 0));
+  if constexpr (A == 0) {
+    *reinterpret_cast<uint4 *>(to) = make_uint4(x[0], x[1], x[2], x[3]);
+  } else {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) to[reg_step<S, A>(m)] = x[m];
+  }
   if constexpr (S < 4) __syncwarp();
   else if constexpr (S == 4) sync_warps(1 + (g >> 6), 64);
   else if constexpr (S == 6) sync_warps(9 + (g >> 8), 256);
   else __syncthreads();
-  get4<B>(buf, x, g);
+  if constexpr (B == 0) {
+    const uint4 u = *reinterpret_cast<const uint4 *>(from);
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+  } else {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) x[m] = from[reg_step<S, B>(m)];
+  }
 }
 __device__ __forceinline__ void round_gs(uint32_t (&x)[4], const RegTwiddles &t, int q) {
   bf_gs(x[0], x[1], t.a[q][0]);
@@ -545,36 +551,35 @@ __device__ __forceinline__ void round_ct(uint32_t (&x)[4], const RegTwiddles &t,
   bf_ct(x[2], x[3], t.a[q][1]);
 }
 
-// Residues in layout 0 in, residues in layout 9 out (without n^-1).  Two buffers of 2048 words, used in turn: a buffer is
-// written again only after a barrier that follows its last reads by every thread sharing the words, here and over calls
-// of the two transforms in turn.
-__device__ __forceinline__ void intt_regs(uint32_t (&x)[4], uint32_t *b0, uint32_t *b1, const RegTwiddles &t, int g) {
+// Residues in layout 0 in, residues in layout 9 out (without n^-1).  `buf`: kRegWords; the two transforms in turn need no
+// barrier between them, two of the same do.
+__device__ __forceinline__ void intt_regs(uint32_t (&x)[4], uint32_t *buf, const RegTwiddles &t, int g) {
   round_gs(x, t, 0);
-  relayout<0, 2>(x, b0, g);
+  relayout<0, 2>(x, buf, g);
   round_gs(x, t, 1);
-  relayout<2, 4>(x, b1, g);
+  relayout<2, 4>(x, buf, g);
   round_gs(x, t, 2);
-  relayout<4, 6>(x, b0, g);
+  relayout<4, 6>(x, buf, g);
   round_gs(x, t, 3);
-  relayout<6, 8>(x, b1, g);
+  relayout<6, 8>(x, buf, g);
   round_gs(x, t, 4);
-  relayout<8, 9>(x, b0, g);
+  relayout<8, 9>(x, buf, g);
   bf_gs(x[0], x[2], t.d);
   bf_gs(x[1], x[3], t.d);
 }
 // 32-bit representatives in layout 9 in, the same in layout 0 out.
-__device__ __forceinline__ void ntt_regs(uint32_t (&x)[4], uint32_t *b0, uint32_t *b1, const RegTwiddles &t, int g) {
+__device__ __forceinline__ void ntt_regs(uint32_t (&x)[4], uint32_t *buf, const RegTwiddles &t, int g) {
   bf_ct(x[0], x[2], t.d);
   bf_ct(x[1], x[3], t.d);
-  relayout<9, 8>(x, b1, g);
+  relayout<9, 8>(x, buf, g);
   round_ct(x, t, 4);
-  relayout<8, 6>(x, b0, g);
+  relayout<8, 6>(x, buf, g);
   round_ct(x, t, 3);
-  relayout<6, 4>(x, b1, g);
+  relayout<6, 4>(x, buf, g);
   round_ct(x, t, 2);
-  relayout<4, 2>(x, b0, g);
+  relayout<4, 2>(x, buf, g);
   round_ct(x, t, 1);
-  relayout<2, 0>(x, b1, g);
+  relayout<2, 0>(x, buf, g);
   round_ct(x, t, 0);
 }
 
@@ -583,7 +588,7 @@ __device__ __forceinline__ void ntt_regs(uint32_t (&x)[4], uint32_t *b0, uint32_
 __global__ void __launch_bounds__(512, 2) offline_rows8_kernel(uint32_t *__restrict__ rows, int count,
                                                                const uint32_t *__restrict__ psi) {
   constexpr int n = 2048;
-  __shared__ __align__(16) uint32_t buf[2 * n];
+  extern __shared__ __align__(16) uint32_t buf[];
   const int g = threadIdx.x;
   RegTwiddles t;
   load_tw(t, psi, g);
@@ -598,7 +603,7 @@ __global__ void __launch_bounds__(512, 2) offline_rows8_kernel(uint32_t *__restr
     if (r + (int)gridDim.x < count)
 #pragma unroll
       for (int m = 0; m < 4; ++m) next[m] = rows[(size_t)(r + gridDim.x) * n + reg_index<9>(g, m)];
-    ntt_regs(x, buf, buf + n, t, g);
+    ntt_regs(x, buf, t, g);
     *reinterpret_cast<uint4 *>(rows + (size_t)r * n + 4 * g) =
         make_uint4(canon_q(x[0]), canon_q(x[1]), canon_q(x[2]), canon_q(x[3]));
     __syncthreads();  // the buffers are free for the next row
@@ -632,7 +637,7 @@ __global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *_
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), k = (int)cl.block_rank();  // one CTA per gadget digit; this CTA's digit
   const int chain = blockIdx.x / C, o = chain >> 1, bar = chain & 1, g = threadIdx.x;
-  uint32_t *b0 = osm, *b1 = osm + n, *wk = osm + 2 * n, *parts = osm + 3 * n;  // parts[buffer][rank][slot]
+  uint32_t *buf = osm, *wk = osm + kRegWords, *parts = wk + n;  // parts[buffer][rank][slot]
   const int shift = bits * k < 32 ? bits * k : 0;
   const uint32_t mask = bits * k < 32 ? (bits >= 32 ? 0xffffffffu : (1u << bits) - 1u) : 0u;
   const uint32_t *evo = ev + (size_t)o * n * n;
@@ -669,10 +674,10 @@ __global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *_
 #pragma unroll
     for (int m = 0; m < 4; ++m)
       agg[m] = (own >> m) & 1u ? __ldg(evo + (size_t)slot_of(e, m) * n + 4 * g + m) : 0u;
-    intt_regs(x, b0, b1, iv, g);
+    intt_regs(x, buf, iv, g);
 #pragma unroll
     for (int m = 0; m < 4; ++m) x[m] = (x[m] >> shift) & mask;
-    ntt_regs(x, b0, b1, fw, g);
+    ntt_regs(x, buf, fw, g);
     uint32_t v[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
