@@ -2057,52 +2057,59 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
       return -4;
     }
   }
-  std::vector<uint32_t> w32(tg * n), v32(tg * n);
+  // One allocation holds the call's scratch, its host inputs first and uploaded together; the hint's aggregates lie in the
+  // packing matrix's own buffer, which the last kernel fills once the walk has read them.
+  const size_t polys = e->rows / n, bt_words = outputs * 2 * (half - 1) * tg * n;
+  size_t need = 0;
+  auto room = [&](size_t bytes) {
+    const size_t at = need;
+    need += round_up(bytes, 256);
+    return at;
+  };
+  const size_t at_psi = room(n * 4), at_psi_inv = room(n * 4), at_w = room(tg * n * 4), at_v = room(tg * n * 4),
+               at_gen = room(half * 2), host_bytes = need;
+  const size_t at_q = room(e->rows * 8), at_qhat = room(e->rows * 4), at_bt = room(bt_words * 4),
+               at_last = room(outputs * 2 * n * 4), at_dft = room(alto::kActWBytes),
+               at_that = room(that ? outputs * tg * n * 4 : 0), at_ahat = room(a_hat ? outputs * n * 4 : 0);
+  std::vector<uint8_t> host(host_bytes);
+  memcpy(host.data() + at_psi, psi.data(), n * 4);
+  memcpy(host.data() + at_psi_inv, psi_inv.data(), n * 4);
+  memcpy(host.data() + at_gen, gen.data(), half * 2);
+  uint32_t *w32 = reinterpret_cast<uint32_t *>(host.data() + at_w), *v32 = reinterpret_cast<uint32_t *>(host.data() + at_v);
   for (size_t i = 0; i < tg * n; ++i) {
     w32[i] = (uint32_t)(w_mask[i] % alto::kQ);
     v32[i] = (uint32_t)(v_mask[i] % alto::kQ);
   }
-  const size_t polys = e->rows / n, bt_words = outputs * 2 * (half - 1) * tg * n;
-  uint64_t *d_q = nullptr;
-  uint32_t *d_qhat = nullptr, *d_psi = nullptr, *d_psi_inv = nullptr, *d_w = nullptr, *d_v = nullptr;
-  uint32_t *d_act = nullptr, *d_bt = nullptr, *d_last = nullptr, *d_that = nullptr, *d_ahat = nullptr;
-  uint16_t *d_gen = nullptr;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   cudaError_t err = cudaSuccess;
   auto step = [&](cudaError_t x) {
     if (err == cudaSuccess) err = x;
   };
+  uint8_t *scratch = nullptr;
   step(cudaEventCreate(&t0));
   step(cudaEventCreate(&t1));
-  step(cudaMalloc(&d_q, e->rows * sizeof(uint64_t)));
-  step(cudaMalloc(&d_qhat, e->rows * sizeof(uint32_t)));
-  step(cudaMalloc(&d_psi, n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_psi_inv, n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_w, tg * n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_v, tg * n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_act, cols * n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_bt, bt_words * sizeof(uint32_t)));
-  step(cudaMalloc(&d_last, outputs * 2 * n * sizeof(uint32_t)));
-  step(cudaMalloc(&d_gen, half * sizeof(uint16_t)));
-  if (that) step(cudaMalloc(&d_that, outputs * tg * n * sizeof(uint32_t)));
-  if (a_hat) step(cudaMalloc(&d_ahat, outputs * n * sizeof(uint32_t)));
-  step(cudaMemcpy(d_q, query, e->rows * sizeof(uint64_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_psi, psi.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_psi_inv, psi_inv.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_w, w32.data(), tg * n * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_v, v32.data(), tg * n * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  step(cudaMemcpy(d_gen, gen.data(), half * sizeof(uint16_t), cudaMemcpyHostToDevice));
+  step(cudaMalloc(&scratch, need));
+  auto words = [&](size_t at) { return reinterpret_cast<uint32_t *>(scratch + at); };
+  uint64_t *d_q = reinterpret_cast<uint64_t *>(scratch + at_q);
+  uint32_t *d_qhat = words(at_qhat), *d_psi = words(at_psi), *d_psi_inv = words(at_psi_inv), *d_w = words(at_w),
+           *d_v = words(at_v), *d_bt = words(at_bt), *d_last = words(at_last);
+  uint32_t *d_that = that ? words(at_that) : nullptr, *d_ahat = a_hat ? words(at_ahat) : nullptr;
+  uint32_t *d_act = reinterpret_cast<uint32_t *>(e->d_ub);  // cols n words of the matrix's cols tg n
+  uint16_t *d_gen = reinterpret_cast<uint16_t *>(scratch + at_gen);
+  uint8_t *d_dft = scratch + at_dft;
+  if (err == cudaSuccess) {
+    step(cudaMemcpy(scratch, host.data(), host_bytes, cudaMemcpyHostToDevice));
+    step(cudaMemcpy(d_q, query, e->rows * sizeof(uint64_t), cudaMemcpyHostToDevice));
+  }
   const size_t act_smem = (1 + alto::kActSmemCols) * n * sizeof(uint32_t), walk_smem = (1 + tg) * n * sizeof(uint32_t);
   step(cudaFuncSetAttribute(alto::offline_act_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)act_smem));
   // n = 2048: the hint on the tensor cores (ALTO_OFFLINE_ACT8=0 runs the shared-memory transforms)
   bool act_mma = n == 2048;
   if (const char *v = getenv("ALTO_OFFLINE_ACT8")) act_mma = act_mma && v[0] != '0';
-  uint8_t *d_dft = nullptr;
   CUtensorMap map_rows, map_dft;
   int sms = 148;
   step(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
   if (act_mma) {
-    step(cudaMalloc(&d_dft, alto::kActWBytes));
     step(cudaFuncSetAttribute(alto::offline_act_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, alto::kActSmem));
     if (err == cudaSuccess && (!make_rows_map(&map_rows, e->d_db, e->db_kbs, e->db_mts, alto::kActCols, 16) ||
                                !make_map(&map_dft, d_dft, 128, 4 * 128, 128, 128)))
@@ -2209,12 +2216,9 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
     if (bold_t_bar)
       step(cudaMemcpy(bold_t_bar + o * per, d_bt + (o * 2 + 1) * per, per * sizeof(uint32_t), cudaMemcpyDeviceToHost));
   }
-  if (that) step(cudaMemcpy(that, d_that, outputs * tg * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-  if (a_hat) step(cudaMemcpy(a_hat, d_ahat, outputs * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-  for (void *x : {(void *)d_q, (void *)d_qhat, (void *)d_psi, (void *)d_psi_inv, (void *)d_w, (void *)d_v,
-                  (void *)d_act, (void *)d_bt, (void *)d_last, (void *)d_gen, (void *)d_that,
-                  (void *)d_ahat, (void *)d_dft})
-    cudaFree(x);
+  if (that && err == cudaSuccess) step(cudaMemcpy(that, d_that, outputs * tg * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+  if (a_hat && err == cudaSuccess) step(cudaMemcpy(a_hat, d_ahat, outputs * n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+  cudaFree(scratch);
   if (t0) cudaEventDestroy(t0);
   if (t1) cudaEventDestroy(t1);
   if (err != cudaSuccess) {

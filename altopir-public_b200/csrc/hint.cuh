@@ -119,14 +119,20 @@ inline bool hint_tables(int n, std::vector<uint32_t> &psi, std::vector<uint32_t>
   const uint32_t root_inv = pow_q(root, kQ32 - 2);
   int logn = 0;
   while ((1 << logn) < n) ++logn;
+  std::vector<uint32_t> pow(n), pow_inv(n);  // root^k, root^-k
+  pow[0] = pow_inv[0] = 1;
+  for (int k = 1; k < n; ++k) {
+    pow[k] = mul_q(pow[k - 1], root);
+    pow_inv[k] = mul_q(pow_inv[k - 1], root_inv);
+  }
   psi.assign(n, 0);
   psi_inv.assign(n, 0);
   for (int k = 0; k < n; ++k) {
     int rev = 0;
     for (int b = 0; b < logn; ++b)
       if (k >> b & 1) rev |= 1 << (logn - 1 - b);
-    psi[k] = pow_q(root, rev);
-    psi_inv[k] = pow_q(root_inv, rev);
+    psi[k] = pow[rev];
+    psi_inv[k] = pow_inv[rev];
   }
   n_inv = inv_pow2_q(logn);
   return true;
