@@ -19,6 +19,9 @@
 // The resident table belongs to the batcher thread alone.  A loopback executor (no engine) answers batches on the
 // host with a deterministic function of the frame; it exists to test queueing and batching without a device.
 #pragma once
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -31,6 +34,29 @@ namespace {
 
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
+}
+
+// Copies a frame into its pool entry (at least 16-byte aligned) with streaming stores: the entry is read next by the copy
+// engine, so that its lines need be neither fetched nor kept.  One thread's submissions are bound by this copy: 48 frames
+// of 2.1 MB and their answers over 16 GiB 19.3 -> 14.4 ms, 60 frames of 197 KB over 128 MiB 1.93 -> 1.48.
+void copy_frame(uint8_t *dst, const uint8_t *src, size_t n) {
+#if defined(__SSE2__)
+  size_t i = 0;
+  for (; i + 64 <= n; i += 64) {
+    const __m128i a = _mm_loadu_si128(reinterpret_cast<const __m128i *>(src + i));
+    const __m128i b = _mm_loadu_si128(reinterpret_cast<const __m128i *>(src + i + 16));
+    const __m128i c = _mm_loadu_si128(reinterpret_cast<const __m128i *>(src + i + 32));
+    const __m128i d = _mm_loadu_si128(reinterpret_cast<const __m128i *>(src + i + 48));
+    _mm_stream_si128(reinterpret_cast<__m128i *>(dst + i), a);
+    _mm_stream_si128(reinterpret_cast<__m128i *>(dst + i + 16), b);
+    _mm_stream_si128(reinterpret_cast<__m128i *>(dst + i + 32), c);
+    _mm_stream_si128(reinterpret_cast<__m128i *>(dst + i + 48), d);
+  }
+  memcpy(dst + i, src + i, n - i);
+  _mm_sfence();
+#else
+  memcpy(dst, src, n);
+#endif
 }
 
 // 64-bit hash of a byte run (multiply-xor over 8-byte words); equal hashes are confirmed by comparing the bytes.
@@ -722,8 +748,8 @@ long long alto_server_submit(void *p, const uint8_t *frame, size_t len) {
   }
   // copy and hash outside the lock: the ticket is not queued yet, so nothing else reads its pool entry
   uint8_t *dst = s->pool + (size_t)t->pool * s->pitch;
-  memcpy(dst, frame, len);
-  const uint64_t key = s->e && len >= 9 + s->ybytes ? key_hash(dst + 9, s->ybytes) : 0;
+  const uint64_t key = s->e && len >= 9 + s->ybytes ? key_hash(frame + 9, s->ybytes) : 0;
+  copy_frame(dst, frame, len);
   {
     std::lock_guard<std::mutex> lk(s->mu);
     t->key = key;
