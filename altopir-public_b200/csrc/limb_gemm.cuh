@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kGemmThreads, GemmShape<BN>::kCtasPerSm)
     int x = (EPI == Epi::kScan ? kb0 - z * args.kb_chunk : kb0) * kBK;
     int s = 0, phase = 1, issued = 0;  // the first round's stages are free
     for (int i = 0; i < nkb; ++i, x += kBK) {
-      if (!mbar_wait(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) break;
+      if (!mbar_wait_warp(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) break;
       const uint32_t sa = base_addr + (uint32_t)s * S::kStageBytes, sb = sa + S::kABytes;
       if (elect_one()) {
         mbar_arrive_expect_tx(full0 + 8 * s, S::kStageBytes);
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kGemmThreads, GemmShape<BN>::kCtasPerSm)
     const uint32_t a0 = desc_lo_sw128(base_addr);
     int s = 0, phase = 0;
     for (int i = 0; i < nkb; ++i) {
-      if (!mbar_wait(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) break;
+      if (!mbar_wait_warp(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) break;
       tc_fence_after();
       const uint32_t a_lo = a0 + (uint32_t)s * (S::kStageBytes >> 4), b_lo = a_lo + (S::kABytes >> 4);
       if (elect_one()) {
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kGemmThreads, GemmShape<BN>::kCtasPerSm)
     // ---------------------------------------------------------------- epilogue (warps 2..5)
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     const int row = q * 32 + lane;
-    const bool ok = mbar_wait(accum, 0, args.err, ALTO_ERR_WAIT_ACCUM, bail);
+    const bool ok = mbar_wait_warp(accum, 0, args.err, ALTO_ERR_WAIT_ACCUM, bail);
     tc_fence_after();
     if (ok) {
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);

@@ -171,7 +171,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       int x = (kb0 - z * args.kb_chunk) * kBK;
       if (EPI == Epi::kPack) x = kb0 * kBK;
       for (int i = 0; i < nkb; ++i, x += kBK) {
-        if (!mbar_wait(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
+        if (!mbar_wait_warp(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
           stop = true;
           break;
         }
@@ -209,10 +209,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
         int m, n, kb0, nkb;
         unit_coords(u, m, n, kb0, nkb);
         const int ab = it % kBufs, use = it / kBufs;
-        if (use > 0 && !mbar_wait(acce0 + 8 * ab, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) break;
+        if (use > 0 && !mbar_wait_warp(acce0 + 8 * ab, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) break;
         const uint32_t d_tmem = tmem_base + (uint32_t)(ab * BN);
         for (int i = 0; i < nkb; ++i) {
-          if (!mbar_wait(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) {
+          if (!mbar_wait_warp(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) {
             stop = true;
             break;
           }
@@ -231,7 +231,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
         if (elect_one()) mma_commit_pair(accf0 + 8 * ab);
         __syncwarp();
       }
-      if (*bail && elect_one()) {
+      if (__any_sync(0xffffffffu, *bail) && elect_one()) {
         // every MMA issued so far completes before this CTA (and its TMEM and shared memory) may go away
         mma_commit_pair(accf0);
         const uint64_t t0 = globaltimer();
@@ -250,7 +250,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       int m, n, kb0, nkb;
       unit_coords(u, m, n, kb0, nkb);
       const int ab = it % kBufs, use = it / kBufs;
-      if (!mbar_wait(accf0 + 8 * ab, use & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) break;
+      if (!mbar_wait_warp(accf0 + 8 * ab, use & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t)(ab * BN) + ((uint32_t)(q * 32) << 16);
       const int grow = m * 256 + (int)rank * 128 + row;
@@ -372,7 +372,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
       int x = (kb0 - z * args.kb_chunk) * kBK;
       if (EPI == Epi::kPack) x = kb0 * kBK;
       for (int i = 0; i < nkb; ++i, x += kBK) {
-        if (!mbar_wait(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
+        if (!mbar_wait_warp(empty0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_EMPTY, bail)) {
           stop = true;
           break;
         }
@@ -414,8 +414,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
         int m, n, kb0, nkb;
         unit_coords(u, m, n, kb0, nkb);
         for (int i = 0; i < nkb; ++i) {
-          if (i == 0 && use > 0 && !mbar_wait(acce0, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) stop = true;
-          if (stop || !mbar_wait(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) {
+          if (i == 0 && use > 0 && !mbar_wait_warp(acce0, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) stop = true;
+          if (stop || !mbar_wait_warp(full0 + 8 * s, (uint32_t)phase, args.err, ALTO_ERR_WAIT_FULL, bail)) {
             stop = true;
             break;
           }
@@ -427,7 +427,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
           }
           __syncwarp();
           if (i == 0 && use > 0) {
-            if (!mbar_wait(acce0 + 8, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) {
+            if (!mbar_wait_warp(acce0 + 8, (use - 1) & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) {
               stop = true;
               break;
             }
@@ -445,7 +445,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
           }
         }
       }
-      if (*bail && elect_one()) {
+      if (__any_sync(0xffffffffu, *bail) && elect_one()) {
         // every MMA issued so far completes before this CTA (and its TMEM and shared memory) may go away
         mma_commit_pair(accf0);
         const uint64_t t0 = globaltimer();
@@ -467,7 +467,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
       const int grow = m * 256 + (int)rank * 128 + row;
       const bool row_ok = grow < args.rows_a;
       for (int t = 0; t < 2; ++t) {
-        if (!mbar_wait(accf0 + 8 * t, use & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) {
+        if (!mbar_wait_warp(accf0 + 8 * t, use & 1, args.err, ALTO_ERR_WAIT_ACCUM, bail)) {
           stop = true;
           break;
         }

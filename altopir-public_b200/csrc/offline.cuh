@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kActThreads, 1)
       for (int k = 0; k < 16; ++k) a0[k] = a1[k] = a2[k] = 0;
       for (int p = 0; p < polys; ++p, ++g) {
         const int b = g & 1, use = g >> 1;
-        mbar_wait(accf0 + 8 * b, use & 1, err, ALTO_ERR_WAIT_ACCUM, bail);
+        mbar_wait_warp(accf0 + 8 * b, use & 1, err, ALTO_ERR_WAIT_ACCUM, bail);
         tc_fence_after();
         const uint32_t ta = tmem + (uint32_t)(b * 4 * N + 16 * c) + ((uint32_t)(q * 32) << 16);
         uint32_t x[16];
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *_
     *reinterpret_cast<uint4 *>(out) = make_uint4(x[0], x[1], x[2], x[3]);
     out -= (size_t)C * n;
     // after a timeout (recorded in *err) the walk goes on, so that every barrier of the block is met by all its threads
-    mbar_wait<true>(bar0 + 8 * pb, (uint32_t)phase, err, ALTO_ERR_WAIT_FULL, &bail);
+    mbar_wait_warp<true>(bar0 + 8 * pb, (uint32_t)phase, err, ALTO_ERR_WAIT_FULL, &bail);
     const uint4 *p = reinterpret_cast<const uint4 *>(parts + (size_t)pb * C * n) + g;
     uint4 u = p[0];
     x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;

@@ -92,6 +92,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
 }
 
+// The same for a converged warp, which waits and goes on as one: false for every lane when any lane gave up, so that no
+// lane is left at a warp-wide instruction after a timeout.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code,
+                                               volatile int *bail) {
+  return __all_sync(0xffffffffu, mbar_wait<CLUSTER>(bar, parity, err, code, bail));
+}
+
 // ------------------------------------------------------------------------------------------------ TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
