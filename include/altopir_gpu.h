@@ -165,7 +165,9 @@ int alto_engine_set_graphs(void *engine, int on);
 
 /* Device time in ms summed over the batches since the last reset, measured with CUDA events on the engine's
  * stream: ms[0] validate, ms[1] limb split + accumulator zeroing, ms[2] scan GEMM, ms[3] pack GEMM, ms[4] tail;
- * *batches receives the number of batches.  Synchronises the engine.  Returns 0, or -4 on a device failure. */
+ * *batches receives the number of batches.  Of a batch that scans in one launch, the scan runs beside the pack: ms[2]
+ * is then what it took beyond the pack's end, and ms[2] + ms[3] the two together; a small batch's preparation is one
+ * kernel, all of it in ms[0].  Synchronises the engine.  Returns 0, or -4 on a device failure. */
 int alto_kernel_times(void *engine, double *ms, long long *batches, int reset);
 
 /* No counterpart in the reference.  alto_answer_device without any device allocation, for callers that cannot
