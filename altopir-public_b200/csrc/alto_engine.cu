@@ -618,13 +618,24 @@ bool pair_kernels_enabled() {
   return !(v && strcmp(v, "single") == 0);
 }
 
+// The longest unit of a scan, in blocks: 256 (exactness), halved down to 64 while the limbs of that many blocks, which the
+// units of all row tiles read one after the other, are more than 16 MB: then they stay in L2 until the last row tile has
+// read them.  8 GiB, ms a batch at units of 256 / 128 / 64 / 32 blocks: 1,024 clients (134 MB at 256) 30.2 / 29.7 / 28.2 /
+// 28.9, 512 14.6 / 14.5 / 14.1 / 14.7, 200 (26 MB) 6.5 / 6.6 / 6.6 / 6.8, 128 3.80 / 3.82 / 3.85.
+int unit_limit(size_t limb_cols) {
+  int p = 256;
+  while (p > 64 && limb_cols * 128 * p > (size_t(16) << 20)) p /= 2;
+  return p;
+}
+
 // The persistent pairs take a launch's units, all of one length, in rounds, so it takes ceil(units / pairs) rounds of a
 // unit's blocks of K plus what a unit costs besides (its epilogue's reductions, the pipeline's refill), `extra` blocks.
 // Finds the split of `kb` blocks over `tiles` tiles with the least sum: returns it in blocks, its blocks per unit in *per.
 // 64 tiles of 256 blocks on 74 pairs (half of a 1 GiB scan, 128 clients): 8 units a tile make 7 rounds of 32 blocks, where
 // twelve units a pair made 7 units a tile, 7 rounds of 37.
-double split_cost(const Engine *e, int kb_chunk, long tiles, int kb, double extra, int *per) {
-  const int pairs = resident_pairs();
+// A unit is at most unit_limit blocks long.
+double split_cost(const Engine *e, size_t limb_cols, int kb_chunk, long tiles, int kb, double extra, int *per) {
+  const int pairs = resident_pairs(), limit = unit_limit(limb_cols);
   double cost = 0;
   *per = 0;
   auto look = [&](int p) {
@@ -636,9 +647,9 @@ double split_cost(const Engine *e, int kb_chunk, long tiles, int kb, double extr
     }
   };
   if (e->nchunks > 1) {  // a unit's blocks divide a record chunk's 256
-    for (int p = kb_chunk; p >= 8; p /= 2) look(p);
+    for (int p = std::min(kb_chunk, limit); p >= 8; p /= 2) look(p);
   } else {
-    const int least = (kb + 255) / 256;
+    const int least = (kb + limit - 1) / limit;
     for (int split = least; split == least || kb / split >= 8; ++split) look((kb + split - 1) / split);
   }
   return cost;
@@ -721,8 +732,8 @@ Plan make_plan(const Engine *e, size_t slots) {
     p.wide_nw = (int)round_up((limb_cols + 2 * p.wide_n - 1) / (2 * p.wide_n), 32);
     const double block_w = 4.0 * p.wide_nw + 180, block_n = 2.0 * p.nw + 100;
     int per;
-    p.wide = split_cost(e, p.kb_chunk, (long)p.scan_m * p.wide_n, p.scan_kb, kWideExtra, &per) * block_w <=
-             split_cost(e, p.kb_chunk, (long)p.scan_m * p.num_n, p.scan_kb, kTileExtra, &per) * block_n;
+    p.wide = split_cost(e, limb_cols, p.kb_chunk, (long)p.scan_m * p.wide_n, p.scan_kb, kWideExtra, &per) * block_w <=
+             split_cost(e, limb_cols, p.kb_chunk, (long)p.scan_m * p.num_n, p.scan_kb, kTileExtra, &per) * block_n;
     auto rounds = [&](long units) { return (double)((units + pairs - 1) / pairs); };
     p.pack_wide = rounds((long)p.pack_m * p.wide_n) * block_w <= rounds((long)p.pack_m * p.num_n) * block_n;
   }
@@ -754,7 +765,7 @@ bool launch_scan(const Engine *e, const Plan &p, const CUtensorMap &map_q, uint3
   if (kb_hi < 0) kb_hi = p.scan_kb;
   int kb_per = p.scan_kb_per;
   if (p.split_each)
-    split_cost(e, p.kb_chunk, (long)mg * p.scan_n, kb_hi - kb_lo, p.wide ? kWideExtra : kTileExtra, &kb_per);
+    split_cost(e, 4 * slots, p.kb_chunk, (long)mg * p.scan_n, kb_hi - kb_lo, p.wide ? kWideExtra : kTileExtra, &kb_per);
   const int splits = (kb_hi - kb_lo + kb_per - 1) / kb_per;
   // The query limbs are re-read by every unit of a K chunk; mark them evict-last only while the whole operand
   // (4 bytes per record and client) is a small part of the 126 MB L2, so stale chunks never crowd it out.

@@ -157,7 +157,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     // ------------------------------------------------------------ TMA producer (both CTAs; the warp, one lane issuing)
     // both CTAs' A tiles and B boxes of this stage: the B box is nw/2 rows (the host makes the map with that box)
     const uint32_t stage_tx = 2u * (uint32_t)(S::kABytes + (nw / 2) * kBK);
-    const uint64_t pol_a = policy_evict_first();
+    const uint64_t pol_a = args.num_n > 1 ? policy_evict_normal() : policy_evict_first();  // as in the wide kernel
     const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
     const uint32_t full_leader0 = map_to_rank(full0, 0);
     int s = 0, phase = 1;  // the first round's stages are free
@@ -358,7 +358,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs; the warp, one lane issuing)
-    const uint64_t pol_a = policy_evict_first();
+    // A tiles that several pairs read, each for its own columns, at about the same time are not the first to leave L2:
+    // evict-first, half a scan of 8 GiB for 1,024 clients read 32.5 GB from DRAM (5.4 without re-reads) and a batch took
+    // 31.8 ms, normal 30; 512 clients 15.0 -> 14.5, 200 6.6 -> 6.5.
+    const uint64_t pol_a = args.num_n > 1 ? policy_evict_normal() : policy_evict_first();
     const uint64_t pol_b = args.b_keep ? policy_evict_last() : policy_evict_normal();
     const uint32_t full_leader0 = map_to_rank(full0, 0);
     int s = 0, phase = 1;  // the first round's stages are free

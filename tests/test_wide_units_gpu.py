@@ -35,3 +35,21 @@ def test_wide_units_return_the_bytes_of_one_tile_units(gpu, oracle, svc, eng, mo
         assert np.array_equal(outs[0][pick], want), b
         assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2]), b
     e.close()
+
+
+@pytest.mark.parametrize("rows,b", [(32768, 129), (32768, 257), (32768 + 9 * 128, 300)])
+def test_scan_units_shortened_for_wide_batches(gpu, oracle, svc, eng, rows, b):
+    """Batches of more than 512 limb columns cut their scan units to 128 or 64 blocks of K (a chunk has 256): one record
+    chunk, and a second one of nine blocks."""
+    p = svc.Params(rows, 2048, n=2048, tg=1) if rows % 2048 == 0 else svc.Params(rows, 96, n=32, tg=4)
+    st = svc.SyntheticState.make(p, seed=rows + b, keep_values=True)
+    st.db_col[::3] = 255
+    e = eng.Engine.from_state(st, threads=svc.threads())
+    req = svc.synthetic_requests(p, b, seed=b)
+    out = np.zeros((b, e.response_len()), dtype=np.uint8)
+    status = np.full(b, -1, dtype=np.int32)
+    assert e.answer([req[i] for i in range(b)], out, status)[0] == b
+    pick = sorted({0, 127, 128, b - 1})
+    _, _, want = oracle.answer(st, [req[i] for i in pick])
+    assert np.array_equal(out[pick], want)
+    e.close()
