@@ -1032,13 +1032,14 @@ int device_groups(const Engine *e, size_t slots) {
 // responses of valid frames to resp + slot * resp_stride.  With the overlapped schedule validation, the query limb
 // split and the zeroing of the scan sums run on the side stream beside the key limb split and the pack, and the
 // tails of all column groups but the last beside the scan (enqueue_scan_tails); the side stream forks from and joins
-// back into the batch's stream, so the batch is complete when its stream passes it.
+// back into the batch's stream, so the batch is complete when its stream passes it.  `ngroups` column groups, or 0 for
+// device_groups; in one group under the overlapped schedule the statuses are in when ev_fork has been passed.
 bool enqueue_batch_direct(Engine *e, Batch *bt, const uint8_t *d_slots, size_t slot_stride, size_t slots,
-                          uint8_t *resp, size_t resp_stride, bool host_status, bool with_marks,
+                          uint8_t *resp, size_t resp_stride, bool host_status, bool with_marks, int ngroups = 0,
                           cudaEvent_t pack_done = nullptr) {
   cudaStream_t st = bt->st;
   const Plan p = make_plan(e, slots);
-  const Groups groups = column_groups(e, p, group_weights(device_groups(e, slots), false));
+  const Groups groups = column_groups(e, p, group_weights(ngroups ? ngroups : device_groups(e, slots), false));
   const bool scan_on_side = e->overlap && groups.count == 1;
   const int bp = (int)round_up(slots, 4);
   int launches = 0;
@@ -1290,14 +1291,15 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
   } while (0)
   if (e->overlap && groups.count == 1 && nc * e->want <= kWholeFrameBytes) {
     // A few small frames upload whole and run as a device batch: the overlap of their uploads with the pack is worth
-    // less than the dozen calls that it takes.
+    // less than the dozen calls that it takes.  In one column group like this path itself, whatever device_groups says,
+    // so that ev_fork lies behind the validation.
     if (stage_ms) ALTO_H(cudaEventRecord(e->ev_begin, st));
     if (!copy_runs(
             nc, e->want, [&](size_t i) { return (const void *)req[cand[i]]; },
             [&](size_t i) { return (void *)(bt->d_req + i * e->slot_stride + kSlotLead); }, cudaMemcpyHostToDevice, st))
       return -4;
     if (stage_ms) ALTO_H(cudaEventRecord(e->ev_keys, st));
-    if (!enqueue_batch_direct(e, bt, bt->d_req, e->slot_stride, nc, bt->d_resp, e->resp_len, true, false,
+    if (!enqueue_batch_direct(e, bt, bt->d_req, e->slot_stride, nc, bt->d_resp, e->resp_len, true, false, 1,
                               stage_ms ? e->ev_pack : nullptr))
       return -4;
     if (stage_ms) ALTO_H(cudaEventRecord(e->ev_group[0], st));
