@@ -1388,6 +1388,7 @@ int answer_host(Engine *e, const uint8_t *const *req, const size_t *len, size_t 
     ++launches;
     if (e->overlap) ALTO_H(cudaEventRecord(bt->ev_qready, vs));
   } else {
+    ALTO_H(cudaStreamWaitEvent(vs, e->ev_keys, 0));  // a batch still in flight on `st` reads and adds into the scan sums
     ALTO_H(cudaMemsetAsync(bt->d_acc, 0, nc * e->cols * sizeof(uint32_t), vs));
     for (int k = 0; k < qgroups; ++k) {
       size_t r0, r1;

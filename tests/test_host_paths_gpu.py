@@ -39,3 +39,47 @@ def test_statuses_of_whole_frames_whatever_the_device_groups(gpu, svc, eng, monk
         assert list(status) == [3 if i == bad else 0 for i in range(b)], bad
         assert np.array_equal(out, expect), bad
     e.close()
+
+
+@pytest.mark.parametrize("groups", ["1", "2"])
+@pytest.mark.parametrize("piped", ["1", str(1 << 40)])
+def test_answer_behind_a_batch_in_flight(gpu, svc, eng, monkeypatch, piped, groups):
+    """alto_answer right behind alto_enqueue_device on the same engine, over two record chunks, with its query words
+    uploaded chunk by chunk and all at once: it waits for the batch's scan sums before it clears them, so both batches
+    return what they return alone."""
+    import torch
+    monkeypatch.setenv("ALTO_PIPED_BYTES", piped)
+    monkeypatch.setenv("ALTO_GROUPS", groups)
+    p = svc.params(65536, 16384)  # 40 frames: 13 MB uploaded, 2.3 MB of responses
+    st = svc.SyntheticState.make(p, seed=71, keep_values=False, host_db=False)
+    e = eng.Engine.from_state(st, threads=svc.threads(), tile=False)
+    ahead, b = 64, 40
+    ql, rl = e.request_len(), e.response_len()
+    stride = (7 + ql + 255) // 256 * 256
+    frames = svc.synthetic_requests(p, ahead + b, seed=72)
+    slots = np.zeros((ahead, stride), dtype=np.uint8)
+    slots[:, 7:7 + ql] = frames[:ahead]
+    slots = torch.from_numpy(slots).cuda()
+    req = [frames[ahead + i] for i in range(b)]
+
+    def enqueue():
+        out = torch.zeros((ahead, rl), dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        e.enqueue_device(slots.data_ptr(), stride, ahead, out.data_ptr(), rl)
+        return out
+
+    def answer():
+        out, status = np.zeros((b, rl), dtype=np.uint8), np.full(b, -1, dtype=np.int32)
+        assert e.answer(req, out, status)[0] == b
+        return out
+
+    first = enqueue()
+    e.sync()
+    want_ahead, want = first.cpu().numpy(), answer()
+    for _ in range(5):
+        out = enqueue()
+        got = answer()
+        e.sync()
+        assert np.array_equal(got, want)
+        assert np.array_equal(out.cpu().numpy(), want_ahead)
+    e.close()
