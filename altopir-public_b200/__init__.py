@@ -70,6 +70,7 @@ def _declare(L):
         "alto_synthetic_db_col": (None, [P, S, S, S, S, I]),
         "alto_synthetic_db_col_device": (I, [P, S, S, S, S]),
         "alto_engine_fill_synthetic": (I, [P]),
+        "alto_engine_set_error": (I, [P, I, c.c_uint32]),
         "alto_hint_ring": (I, [P, P, P, I]),
         "alto_engine_offline": (I, [P, P, P, P, P, P, P, P, c.POINTER(c.c_double)]),
         "alto_synthetic_requests_device": (I, [P, S, S, S, S, S, U64, U64]),
@@ -96,7 +97,7 @@ EXPORTS = (
     "alto_engine_free", "alto_request_len", "alto_response_len", "alto_answer", "alto_last_error",
     "alto_answer_device", "alto_last_launches", "alto_enqueue_device", "alto_engine_sync", "alto_engine_stream",
     "alto_kernel_times", "alto_engine_set_graphs", "alto_engine_set_lanes", "alto_engine_fence",
-    "alto_engine_set_tuning", "alto_answer_device_noalloc",
+    "alto_engine_set_error", "alto_engine_set_tuning", "alto_answer_device_noalloc",
     "alto_answer_device_parts", "alto_ipc_export", "alto_ipc_import", "alto_ipc_release", "alto_server_new",
     "alto_server_new_keyed", "alto_server_log",
     "alto_server_new_loopback",

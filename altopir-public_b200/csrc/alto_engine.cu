@@ -1195,6 +1195,14 @@ bool check_batch_error(Batch *b) {
   return true;
 }
 
+// Clears a batch's error word for work that reports its own timeouts in it, and puts back at the end what was there: the
+// code of an earlier batch stays alto_engine_sync's to report.  Nothing else may run on the batch meanwhile.
+struct ErrorSetAside {
+  uint32_t *word, earlier;
+  explicit ErrorSetAside(Batch *b) : word(b->h_err), earlier(*b->h_err) { *word = 0; }
+  ~ErrorSetAside() { *word = earlier; }
+};
+
 // The same for the main batch, then the pending timing marks folded into the totals.
 bool check_error_word(Engine *e) { return check_batch_error(&e->main) && accumulate_pending(e); }
 
@@ -1897,6 +1905,14 @@ int alto_engine_sync(void *p) {
   return sync_engine(e) ? 0 : -4;
 }
 
+int alto_engine_set_error(void *p, int lane, uint32_t code) {
+  Engine *e = static_cast<Engine *>(p);
+  if (!e || lane < 0 || lane >= e->lanes_made || !code || code > 15) return -1;
+  if (cudaSetDevice(e->dev) != cudaSuccess || cudaStreamSynchronize(lane_batch(e, lane)->st) != cudaSuccess) return -4;
+  *lane_batch(e, lane)->h_err |= code;
+  return 0;
+}
+
 void *alto_engine_stream(void *p) { return p ? static_cast<void *>(static_cast<Engine *>(p)->main.st) : nullptr; }
 
 int alto_kernel_times(void *p, double *ms, long long *batches, int reset) {
@@ -2071,6 +2087,7 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
       return -4;
     }
   }
+  ErrorSetAside aside(&e->main);
   // One allocation holds the call's scratch, its host inputs first and uploaded together; the hint's aggregates lie in the
   // packing matrix's own buffer, which the last kernel fills once the walk has read them.
   const size_t polys = e->rows / n, bt_words = outputs * 2 * (half - 1) * tg * n;

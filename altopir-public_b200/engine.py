@@ -231,6 +231,11 @@ class Engine:
         if r < 0:
             raise EngineError(f"engine error {r}: {last_error()}")
 
+    def set_error(self, code, lane=0):
+        """alto_engine_set_error: `code` left in the lane's error word, as a kernel whose wait ran out does."""
+        if lib().alto_engine_set_error(self.ptr, lane, code) < 0:
+            raise EngineError(f"cannot set error {code} of lane {lane}")
+
     def stream(self):
         """The engine's cudaStream_t as an integer handle (torch.cuda.ExternalStream accepts it)."""
         return lib().alto_engine_stream(self.ptr)

@@ -144,6 +144,11 @@ int alto_engine_sync(void *engine);
 int alto_engine_set_lanes(void *engine, int lanes);
 int alto_engine_fence(void *engine);
 
+/* Leaves `code` (1 to 15, the bits of the kernels' bounded waits) in the error word of lane `lane` (0 <= lane < lanes set
+ * so far), as a kernel whose wait ran out does, once that lane's batches are done: for tests of what a caller is told
+ * about a batch that failed, which need no fault on the device.  0, -1 for bad arguments or -4. */
+int alto_engine_set_error(void *engine, int lane, uint32_t code);
+
 /* The cudaStream_t the engine launches its kernels on (for events and stream ordering in the caller). */
 void *alto_engine_stream(void *engine);
 
@@ -309,9 +314,9 @@ int alto_hint_ring(void *engine, const uint64_t *query, uint64_t *out, int perm_
  * unity; gadget digits of floor(32 / tg) + 1 bits.  Optional host outputs (NULL to skip), all u32 in [0, q):
  * bold_t and bold_t_bar, outputs x (n/2 - 1) x tg x n each; that (bold_t_hat), outputs x tg x n; a_hat, outputs x n.
  * ms (optional) receives the device time of the set-up.  Waits for the engine's batches in flight (a serving loop
- * must not run on the engine meanwhile); allocates about 4 tg n cols + 12 records bytes of device scratch for the call
- * (1.1 GB at 32 KB records, n = 2048, tg = 4).  0, -1 for bad arguments or an unsupported
- * configuration (the engine is untouched), -4 for a device failure (the engine's packing state is then undefined:
+ * must not run on the engine meanwhile), whose errors stay for alto_engine_sync to report; allocates about
+ * 4 tg n cols + 12 records bytes of device scratch for the call (1.1 GB at 32 KB records, n = 2048, tg = 4).
+ * 0, -1 for bad arguments or an unsupported configuration (the engine is untouched), -4 for a device failure (the engine's packing state is then undefined:
  * call again or free it). */
 int alto_engine_offline(void *engine, const uint64_t *query, const uint64_t *w_mask, const uint64_t *v_mask,
                         uint32_t *bold_t, uint32_t *bold_t_bar, uint32_t *that, uint32_t *a_hat, double *ms);
