@@ -29,6 +29,7 @@
 #include "kernels.cuh"
 #include "modq.cuh"
 #include "sm100.cuh"
+#include "waits.cuh"
 
 namespace alto {
 
@@ -665,9 +666,9 @@ __global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *_
   }
   uint32_t *out = bt + (((size_t)chain * (half - 1) + (half - 2)) * C + k) * n + 4 * g;
   cluster_sync_all();  // w is in shared memory, and every CTA's barriers are ready for the others' shares
-  int pb = 0, phase = 0;
+  ShareTurns turn;  // the same in all threads of a warp
   for (int i = half - 2; i >= 0; --i) {
-    if (g == 0) mbar_arrive_expect_tx(bar0 + 8 * pb, (uint32_t)((C - 1) * n * 4));
+    if (g == 0) turn.arm([&](int b) { mbar_arrive_expect_tx(bar0 + 8 * b, (uint32_t)((C - 1) * n * 4)); });
     // the aggregates are gathered now, so that their latency hides behind the transforms
     e = (e * 0xcccccccdu) & (2 * n - 1);  // times 5^-1 mod 2n
     uint32_t agg[4];
@@ -685,19 +686,23 @@ __global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *_
       v[m] = mont_q(x[m], wk[slot_of(e, m)]);
       if ((own >> m) & 1u) v[m] = add_q(v[m], mont_q(agg[m], agg_scale));
     }
-    uint32_t *mine = parts + (size_t)(pb * C + k) * n;
+    uint32_t *mine = parts + (size_t)(turn.buf * C + k) * n;
     reinterpret_cast<uint4 *>(mine)[g] = make_uint4(v[0], v[1], v[2], v[3]);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    if ((g & 31) < C && (g & 31) != k) {  // each warp sends its 128 words as soon as they are written
-      const uint32_t src = smem_u32(mine + 4 * (g & ~31)), r = (uint32_t)(g & 31);
-      bulk_copy_to_cta(map_to_rank(src, r), src, 512, map_to_rank(bar0 + 8 * pb, r));
-    }
+    if ((g & 31) < C && (g & 31) != k)  // each warp sends its 128 words as soon as they are written
+      turn.send([&](int b) {
+        const uint32_t src = smem_u32(mine + 4 * (g & ~31)), r = (uint32_t)(g & 31);
+        bulk_copy_to_cta(map_to_rank(src, r), src, 512, map_to_rank(bar0 + 8 * b, r));
+      });
     *reinterpret_cast<uint4 *>(out) = make_uint4(x[0], x[1], x[2], x[3]);
     out -= (size_t)C * n;
-    // after a timeout (recorded in *err) the walk goes on, so that every barrier of the block is met by all its threads
-    mbar_wait_warp<true>(bar0 + 8 * pb, (uint32_t)phase, err, ALTO_ERR_WAIT_FULL, &bail);
-    const uint4 *p = reinterpret_cast<const uint4 *>(parts + (size_t)pb * C * n) + g;
+    // after a timeout (recorded in *err) the walk goes on by itself, so that every barrier of the block is met by all its
+    // threads
+    turn.wait([&](int b, uint32_t parity) {
+      return mbar_wait_warp<true>(bar0 + 8 * b, parity, err, ALTO_ERR_WAIT_FULL, &bail);
+    });
+    const uint4 *p = reinterpret_cast<const uint4 *>(parts + (size_t)turn.buf * C * n) + g;
     uint4 u = p[0];
     x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
     for (int r = 1; r < C; ++r) {
@@ -706,9 +711,14 @@ __global__ void __launch_bounds__(512, 1) offline_walk8_kernel(const uint32_t *_
     }
 #pragma unroll
     for (int m = 0; m < 4; ++m) x[m] = canon_q(x[m]);
-    pb ^= 1;
-    phase ^= pb ^ 1;  // each barrier's phases alternate
+    turn.next();
   }
+  if (!turn.live) {  // copies already issued land within microseconds; no CTA is gone before
+    const uint64_t t0 = globaltimer();
+    while (globaltimer() - t0 < 200000ull) {
+    }
+  }
+  __syncwarp();
   cluster_sync_all();  // no CTA exits while another may still copy into its shared memory
   if (k == 0)
 #pragma unroll

@@ -1,0 +1,19 @@
+"""What follows from a bounded wait that ran out, on the host: no kernel runs and no wait runs out on a device."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "altopir-public_b200", "csrc")
+
+
+def test_exchange_of_shares_after_a_lost_share(tmp_path):
+    cxx = shutil.which("g++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path / "waits")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-I", CSRC, os.path.join(HERE, "cpp", "test_waits.cpp"), "-o", exe],
+                   check=True)
+    assert subprocess.run([exe], capture_output=True, text=True, timeout=300).stdout.strip() == "0"
