@@ -416,7 +416,7 @@ void free_scratch(Batch *b) {
   b->cap = 0;
 }
 
-// Stream, error word and its pinned mirror of a batch (scratch comes later, on demand).
+// Streams, events and error word of a batch (scratch comes later, on demand).
 bool init_batch(Batch *b, bool timing) {
   // The batch's stream has the highest priority and the side stream the lowest, so that when a GEMM and a tail are
   // both waiting for SMs the GEMM's persistent CTAs are placed first and the tail's CTAs take the room left beside
@@ -1184,7 +1184,7 @@ bool copy_runs(size_t items, size_t width, SrcAt src_at, DstAt dst_at, cudaMemcp
 // error word.
 // After a batch's stream has been waited for: false (and the word reset) when a kernel wait timed out.
 bool check_batch_error(Batch *b) {
-  const uint32_t err = *b->h_err;
+  const uint32_t err = alto::error_codes(*b->h_err);
   if (err) {
     *b->h_err = 0;
     char buf[96];
@@ -1909,7 +1909,8 @@ int alto_engine_set_error(void *p, int lane, uint32_t code) {
   Engine *e = static_cast<Engine *>(p);
   if (!e || lane < 0 || lane >= e->lanes_made || !code || code > 15) return -1;
   if (cudaSetDevice(e->dev) != cudaSuccess || cudaStreamSynchronize(lane_batch(e, lane)->st) != cudaSuccess) return -4;
-  *lane_batch(e, lane)->h_err |= code;
+  for (uint32_t bit = 1; bit <= 8; bit <<= 1)
+    if (code & bit) alto::record_error(lane_batch(e, lane)->h_err, bit);
   return 0;
 }
 

@@ -6,17 +6,11 @@
 #include <cuda.h>
 #include <cstdint>
 
+#include "waits.cuh"
+
 #ifndef ALTO_WAIT_NS
 #define ALTO_WAIT_NS 2000000000ull  // 2 s: far above any legitimate wait (a whole batch takes milliseconds)
 #endif
-
-// Error codes written to the error word, which is pinned host memory (a plain store; the last one stays).
-enum : uint32_t {
-  ALTO_ERR_WAIT_FULL = 1u,    // MMA issuer gave up waiting for a TMA stage
-  ALTO_ERR_WAIT_EMPTY = 2u,   // producer gave up waiting for a stage to be released
-  ALTO_ERR_WAIT_ACCUM = 4u,   // epilogue gave up waiting for the accumulator
-  ALTO_ERR_WAIT_DRAIN = 8u,   // a bail-out drain wait gave up
-};
 
 namespace alto {
 
@@ -72,7 +66,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
   return ok != 0;
 }
-// Waits for the phase with the given parity to complete.  Returns false (and ORs `code` into *err) after
+// Waits for the phase with the given parity to complete.  Returns false (and records `code` in *err) after
 // ALTO_WAIT_NS of wall time, or at once when another role of this CTA has already recorded an error.
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code,
@@ -84,7 +78,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     if ((it & 63u) == 63u) {
       if (*bail) return false;
       if (globaltimer() - t0 > ALTO_WAIT_NS) {
-        *reinterpret_cast<volatile uint32_t *>(err) = code;
+        record_error(err, code);
         *bail = 1;
         return false;
       }

@@ -5,7 +5,27 @@
 
 #include "modq.cuh"
 
+// What ran out, as recorded in a batch's error word.
+enum : uint32_t {
+  ALTO_ERR_WAIT_FULL = 1u,    // MMA issuer gave up waiting for a TMA stage
+  ALTO_ERR_WAIT_EMPTY = 2u,   // producer gave up waiting for a stage to be released
+  ALTO_ERR_WAIT_ACCUM = 4u,   // epilogue gave up waiting for the accumulator
+  ALTO_ERR_WAIT_DRAIN = 8u,   // a bail-out drain wait gave up
+};
+
 namespace alto {
+
+// The error word is pinned host memory, which the CTAs of a batch write without atomics: every code has a byte of its own,
+// so that none hides another.  error_codes: the codes recorded in a word, together.
+ALTO_HD void record_error(uint32_t *word, uint32_t code) {
+  volatile uint8_t *byte = reinterpret_cast<volatile uint8_t *>(word);
+  byte[code == ALTO_ERR_WAIT_FULL ? 0 : code == ALTO_ERR_WAIT_EMPTY ? 1 : code == ALTO_ERR_WAIT_ACCUM ? 2 : 3] = 1;
+}
+ALTO_HD uint32_t error_codes(uint32_t word) {
+  uint32_t codes = 0;
+  for (int i = 0; i < 4; ++i) codes |= (uint32_t)((word >> (8 * i) & 0xffu) != 0) << i;
+  return codes;
+}
 
 // One warp's part, step by step, in an exchange through two buffers with a barrier each, used in turn (the walk of
 // offline.cuh): one thread of the CTA arms the step's barrier for the shares of the other CTAs, every warp sends its own,

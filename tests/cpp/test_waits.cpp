@@ -1,5 +1,6 @@
 // The walk's exchange of shares (ShareTurns, waits.cuh) on a model of its mbarriers, with a share that never arrives: every
 // CTA's steps come to an end, no barrier is armed that expects no arrival, and none counts more bytes than it can hold.
+// With an argument: the codes of an error word.
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -71,7 +72,27 @@ bool walk(int C, int W, int steps, int from, int to, int w, int at, int *live) {
   return good;
 }
 
-int main() {
+// Every set of codes, recorded in any order and more than once, is the set that is read.
+static int codes() {
+  int bad = 0;
+  for (uint32_t set = 0; set < 16; ++set)
+    for (int last = 0; last < 4; ++last) {
+      uint32_t word = 0;
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t bit = 1u << ((last + 1 + i) % 4);
+        if (set & bit) record_error(&word, bit);
+      }
+      bad += error_codes(word) != set || (set != 0) != (word != 0);
+    }
+  return bad;
+}
+
+int main(int argc, char **) {
+  if (argc > 1) {
+    const int bad = codes();
+    printf("%d\n", bad);
+    return bad != 0;
+  }
   int bad = 0, live = 0;
   for (int C : {2, 3, 4, 8}) {
     const int W = 16, steps = 1023;

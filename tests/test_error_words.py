@@ -32,3 +32,18 @@ def test_offline_setup_leaves_an_earlier_batchs_error_to_sync(gpu, svc, eng):
         with pytest.raises(eng.EngineError):
             e.set_error(code, lane)
     e.close()
+
+
+@pytest.mark.gpu
+def test_every_recorded_code_is_reported(gpu, svc, eng):
+    """Two waits that ran out in one batch are both named; another lane's word is its own."""
+    p = svc.params(2048, 2048)
+    e = eng.Engine.from_state(svc.SyntheticState.make(p, seed=3))
+    e.set_lanes(2)
+    e.set_error(1)
+    e.set_error(8)
+    e.set_error(2, 1)
+    with pytest.raises(eng.EngineError, match="0x9"):  # the main lane is looked at last
+        e.sync()
+    e.sync()
+    e.close()
