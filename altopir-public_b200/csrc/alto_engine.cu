@@ -307,7 +307,8 @@ struct Engine {
   std::atomic<int> last_launches{0};  // written by whichever thread enqueued the latest batch (a serving loop's too)
   bool use_graphs = false;  // replay captured launch sequences (alto_engine_set_graphs)
   bool overlap = true;      // the two-stream schedule of a batch (ALTO_OVERLAP=0 runs it on one stream)
-  int groups = 0;           // column groups of the scan and tail of a device batch (ALTO_GROUPS: 1 to 8; 0: device_groups)
+  // column groups of the scan and tail of a device batch (ALTO_GROUPS): 1 to 8 for every batch, 0 by its size (device_groups)
+  int groups = 0;
   // The column groups of alto_answer, whose downloads overlap the scan, as weights (ALTO_HOST_WEIGHTS, or
   // ALTO_HOST_GROUPS groups with a last one of half the size).  A group's side-stream tail runs once the next group's
   // scan has left the SMs; the tails of the last host_inline groups before the last run on the batch's stream
@@ -1015,15 +1016,16 @@ bool enqueue_scan_tails(Engine *e, Batch *bt, const Plan &p, const CUtensorMap &
   return true;
 }
 
-// Column groups of a device batch.  One, with the preparation in one launch and the scan on the side stream without
+// Column groups of a device batch: ALTO_GROUPS where it is given.  Otherwise one, with the preparation in one launch and the scan on the side stream without
 // waiting for the pack (its units fill the SMs as the pack's run out, instead of starting on an idle device), unless the
 // query split is long enough to be worth hiding beside the pack, or the tails enough to be worth hiding beside the scan:
 // then two, the first one's tails beside the second one's scan.  us a call, two groups / one: 1 GiB, one client 376 / 336,
 // 128 clients 856 / 845, four batches of 128 on two lanes 3,345 / 3,310; 8 GiB, 100 clients (105 MB of query words)
 // 3,094 / 3,115.
 int device_groups(const Engine *e, size_t slots) {
-  if (!e->overlap || slots * e->resp_len < kGroupedRespBytes) return 1;
+  if (!e->overlap) return 1;
   if (e->groups) return e->groups;
+  if (slots * e->resp_len < kGroupedRespBytes) return 1;
   return 4 * slots * e->rows > kHiddenSplitBytes || slots * e->resp_len > kHiddenTailBytes ? 2 : 1;
 }
 
@@ -1588,7 +1590,7 @@ void *create_engine(const uint8_t *db_col, size_t ld, size_t rows, size_t cols, 
   }
   if ((err = cudaStreamCreateWithFlags(&e->st_copy, cudaStreamNonBlocking)) != cudaSuccess) return fail("stream", err);
   if (const char *v = getenv("ALTO_OVERLAP")) e->overlap = v[0] != '0';
-  if (const char *v = getenv("ALTO_GROUPS")) e->groups = std::max(1, std::min(8, atoi(v)));
+  if (const char *v = getenv("ALTO_GROUPS")) e->groups = std::max(0, std::min(8, atoi(v)));
   if (const char *v = getenv("ALTO_HOST_GROUPS")) e->host_weights = group_weights(atoi(v), true);
   if (const char *v = getenv("ALTO_HOST_INLINE")) e->host_inline = std::max(0, std::min(7, atoi(v)));
   if (const char *v = getenv("ALTO_PIPED_BYTES")) e->piped_bytes = (size_t)strtoull(v, nullptr, 10);

@@ -83,3 +83,39 @@ def test_answer_behind_a_batch_in_flight(gpu, svc, eng, monkeypatch, piped, grou
         assert np.array_equal(got, want)
         assert np.array_equal(out.cpu().numpy(), want_ahead)
     e.close()
+
+
+def test_column_groups_of_the_device_path_follow_the_setting(gpu, svc, eng, monkeypatch):
+    """ALTO_GROUPS: a count holds for small batches too; 0 is the choice by size, as without the variable, which takes one
+    launch of the scan for a small batch and two for one of more than 32 MB of responses."""
+    import torch
+    p = svc.params(2048, 32768)  # 16 response parts of 7 KB
+    st = svc.SyntheticState.make(p, seed=81, keep_values=False, host_db=False)
+    launches, outs = {}, {}
+    small, large = 3, 300
+    for setting in (None, "0", "1", "2", "4", "-3", "many"):
+        monkeypatch.delenv("ALTO_GROUPS", raising=False)
+        if setting is not None:
+            monkeypatch.setenv("ALTO_GROUPS", setting)
+        e = eng.Engine.from_state(st, threads=svc.threads(), tile=False)
+        ql, rl = e.request_len(), e.response_len()
+        assert small * rl < 2 << 20 and large * rl > 32 << 20
+        stride = (7 + ql + 255) // 256 * 256
+        slots = torch.zeros((large, stride), dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        svc.synthetic_requests_device(p, large, 82, slots.data_ptr(), stride)
+        for b in (small, large):
+            out = torch.zeros((b, rl), dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            assert e.answer_device(slots.data_ptr(), stride, b, out.data_ptr(), rl, np.zeros(b, dtype=np.int32)) == b
+            launches[setting, b] = e.last_launches()
+            outs[setting, b] = out.cpu().numpy()
+        e.close()
+    for setting in ("0", "-3", "many"):
+        for b in (small, large):
+            assert launches[setting, b] == launches[None, b], (setting, b)
+    for b in (small, large):
+        assert launches["1", b] == 4 and launches["2", b] == 8 and launches["4", b] == 12, (b, launches)
+        for setting in ("0", "1", "2", "4", "-3", "many"):
+            assert np.array_equal(outs[setting, b], outs[None, b]), (setting, b)
+    assert launches[None, small] == 4 and launches[None, large] == 8
