@@ -2067,8 +2067,8 @@ int alto_engine_offline(void *p, const uint64_t *query, const uint64_t *w_mask, 
   const size_t n = e->n, tg = e->tg, cols = e->cols, outputs = e->outputs, half = n / 2;
   std::vector<uint32_t> psi, psi_inv;
   uint32_t n_inv = 0;
-  if (n < 8 || e->rows % n || e->row1_off % n || !alto::hint_tables((int)n, psi, psi_inv, n_inv)) {
-    set_error("alto_engine_offline: needs n a power of two in [8, 2048], records a multiple of n, row 1 at q2_bits n");
+  if (n < (size_t)alto::kPlaneMinN || e->rows % n || e->row1_off % n || !alto::hint_tables((int)n, psi, psi_inv, n_inv)) {
+    set_error("alto_engine_offline: needs n a power of two in [16, 2048], records a multiple of n, row 1 at q2_bits n");
     return -1;
   }
   const int q2_bits = (int)(e->row1_off / n);

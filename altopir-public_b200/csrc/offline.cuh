@@ -789,7 +789,8 @@ __global__ void __launch_bounds__(1024) offline_finish_kernel(const uint32_t *__
 // scatters each to its slot s in shared memory, then writes 32 rows of the matrix, 4 KB together in every tile.  Bound by
 // HBM and the scattered shared-memory stores: the 1 GiB matrix takes 0.61 ms (1 GiB read, 1 GiB written; 0.33 at the copy
 // rate) against 2.47 with one thread per value, a 32-byte sector read for each and four byte stores.
-constexpr int kPlaneCols = 8;
+// It writes 16 slots at a time, so n is at least 16 (a multiple of it, being a power of two).
+constexpr int kPlaneCols = 8, kPlaneMinN = 16;
 __global__ void __launch_bounds__(256) offline_planes_kernel(const uint32_t *__restrict__ bt, int n, int logn, int tg,
                                                              const uint16_t *__restrict__ gen, uint32_t tail_scale,
                                                              uint8_t *__restrict__ ub, size_t kbs) {
