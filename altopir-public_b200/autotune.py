@@ -19,15 +19,16 @@ sys.path.insert(0, os.path.dirname(HERE))
 BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256, 512, 1024)
 
 
-def candidates(b, nchunks):
+def candidates(b):
+    """Plans (pair, wide, bn_cap, units_per_pair) for batches of b.  Above 256 limb columns the engine has wide units and
+    splits the scan by rounds of units (units_per_pair 0); below, 0 is its fixed target of 12."""
     limb_cols = 4 * ((b + 3) // 4 * 4)
     out = [(0, -1, 0, 0)]  # single-CTA kernels
     if limb_cols > 16:
         caps = (256, 128) if limb_cols > 128 else (256,)
         for cap in caps:
-            wides = (0, 1) if cap == 256 and limb_cols >= 512 else (0,)
-            for wide in wides:
-                for upp in (6, 12, 24):
+            for wide in (0, 1) if cap == 256 and limb_cols > 256 else (0,):
+                for upp in (0, 6, 12, 24) if limb_cols > 256 else (6, 12, 24):
                     out.append((1, wide, cap, upp))
     return out
 
@@ -70,7 +71,6 @@ def main():
         st = svc.SyntheticState.make(p, seed=5, keep_values=False, host_db=False)  # database made on the device
         e = eng.Engine.from_state(st, threads=svc.threads(), tile=False)
         e.set_tuning([])
-        nchunks = (rows + 32767) // 32768
         bmax = max(buckets)
         ql, rl = e.request_len(), e.response_len()
         stride = (7 + ql + 255) // 256 * 256
@@ -84,7 +84,7 @@ def main():
             want = d_out[:b].clone()
             t_est = time_plan(torch, e, slots, stride, b, d_out, rl, 2)
             iters = max(2, int(a.budget_ms / max(t_est, 1e-3)))
-            plans = [None] + candidates(b, nchunks)   # None: the built-in plan
+            plans = [None] + candidates(b)   # None: the built-in plan
             times = {i: [] for i in range(len(plans))}
             for _ in range(a.rounds):                 # interleaved rounds: clock and power drift hit all plans alike
                 for i, plan in enumerate(plans):
