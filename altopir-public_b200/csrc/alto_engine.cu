@@ -266,9 +266,10 @@ void clear_graphs(Batch *b) {
 struct TuneEntry {
   int b_max;
   int pair;            // 1 CTA-pair kernels, 0 single-CTA kernels, -1 pairs when a batch has > 16 limb columns
-  int wide;            // 1 wide scan units where possible, 0 never, -1 for databases of several record chunks
+  int wide;            // 1 wide scan units above 256 limb columns, 0 never, -1 by make_plan's estimate of rounds
   int bn_cap;          // largest limb-column tile of the pair kernels (32..256), 0 = 256
-  int units_per_pair;  // scan split target: units per resident CTA pair, 0 = 12
+  int units_per_pair;  // scan split target: units per resident CTA pair; 0 = by rounds (split_cost) above 256 limb
+                       // columns, 12 below
 };
 
 struct Engine {
@@ -1182,8 +1183,6 @@ bool copy_runs(size_t items, size_t width, SrcAt src_at, DstAt dst_at, cudaMemcp
   return true;
 }
 
-// Waits for the engine's stream, folds pending timing marks into the totals and checks (then clears) the device
-// error word.
 // After a batch's stream has been waited for: false (and the word reset) when a kernel wait timed out.
 bool check_batch_error(Batch *b) {
   const uint32_t err = alto::error_codes(*b->h_err);

@@ -47,7 +47,7 @@ struct PairArgs {
   int clients;      // valid clients
   int cols;         // record bytes: row stride of the outputs
   uint32_t *out;    // scan: acc[c * cols + col] (pre-zeroed, summed mod 2^32); pack: beta[c * cols + col]
-  uint32_t *err;    // device error word
+  uint32_t *err;    // the batch's error word
   int b_keep;       // 1: keep the B operand in L2 (evict_last; it is small and read by every unit), 0: normal
   int kb_chunk;     // scan: 128-byte blocks per record chunk of the 3-D query-limb map (units never straddle chunks)
   int m_begin;      // first 256-row tile along A (a launch may cover a column group)

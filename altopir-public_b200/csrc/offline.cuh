@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) offline_act_kernel(const uint8_t *__restr
 // zeta_i' = psi[128 + i']^2 (Cooley-Tukey stages over psi^brv), so its coefficient r is sum_j W[i'][j] x[16 j + r] with
 // W[i'][j] = zeta_i'^j: a 128 x 128 matrix of four byte limbs times the records' bytes, exact in int32 (128 x 255 x 255 <
 // 2^23).  A thread then holds the 16 coefficients of one block of one column, so the other four stages, the product with
-// qhat and the sum over p stay in its registers and nothing is exchanged.
+// qhat and the sum over p are that thread's own and nothing is exchanged.
 //
 // Operands.  A = the limbs of W, 128 rows x 128 bytes K-major with 128-byte swizzling, resident in shared memory.  B =
 // kActCols columns of the database for one p, N = (column, r), K = j: a tile row (one column, 128 records) holds eight j
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256) offline_act_kernel(const uint8_t *__restr
 //
 // Persistent, one CTA an SM: warps 0..15 transform (warp w: TMEM lanes 32 (w & 3).., column w >> 2), warp 16 loads, warp
 // 17 issues the MMAs.  Bound by the 16 warps' integer work (53 instructions a record byte, the multiplier pipe 78 %
-// busy; the tensor pipe 10 %).  Measured: 2.2 ms a GiB of database, against 8.9 with all eleven stages in registers and
+// busy; the tensor pipe 10 %).  18 warps leave 96 registers a thread, a few short: ptxas spills 132 bytes.  Measured: 2.2 ms a GiB of database, against 8.9 with all eleven stages in registers and
 // one shared-memory exchange every three of them.
 constexpr int kActCols = 4;                            // database columns of a unit
 constexpr int kActStageBytes = 16 * kActCols * 128;    // one p of a unit: 16 tiles x kActCols rows
@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(kActThreads, 1)
           mac96(a0[4 * v + 3], a1[4 * v + 3], a2[4 * v + 3], x[4 * v + 3], y.w);
         }
       }
-      // 2^32 = 12287 and 2^64 = 12287^2 (mod Q); a2 < 2^32 / 12287^2 products
+      // 2^32 = 12287 and 2^64 = 12287^2 (mod Q).  a2 counts at most one carry a product (polys < 2^31 of them), so the sum
+      // stays below 2^59
 #pragma unroll
       for (int k = 0; k < 16; ++k)
         stage_out[(k * 128 + i) * kActCols + c] =

@@ -1,7 +1,7 @@
 // sm100.cuh -- thin inline-PTX layer for the Blackwell (sm_100a) primitives the answer engine uses:
 // mbarriers with bounded waits, TMA tiled loads, tcgen05 TMEM allocation, tcgen05.mma kind::i8, tcgen05.commit
 // and tcgen05.ld.  Every wait in this file gives up after ALTO_WAIT_NS nanoseconds of wall time, records an error
-// code in the engine's device error word and returns false, so that a lost arrival can never hang the GPU.
+// code in the batch's error word (waits.cuh) and returns false, so that a lost arrival can never hang the GPU.
 #pragma once
 #include <cuda.h>
 #include <cstdint>

@@ -79,7 +79,8 @@ size_t alto_response_len(const void *engine);
  * whose responses download while the next group computes.  A few small frames (2 MB in all) upload whole instead and
  * their scan runs beside the pack.  When stage_ms is not NULL it receives device times in
  * ms: [0] header and y-key upload, [1] validation, query split, scans and tails, [2] key split and pack, [3] the
- * last group's download.
+ * last group's download; of frames uploaded whole [0] their upload, [1] what scan and tail took beyond the pack's end,
+ * [2] validation, both splits and the pack, [3] the download.
  * Returns the number of valid requests, -1 for bad arguments, -3 when the tail parameters are invalid (n not a
  * power of two >= 16, q1 >= 2^21, q1_bits > 24, n % 8, or row 1 not fitting in part_len), -4 when the device
  * failed (CUDA error or a kernel wait that timed out; alto_last_error() has the reason).  Calls on one engine must
@@ -154,8 +155,8 @@ void *alto_engine_stream(void *engine);
 
 /* Tuning table of this engine: n entries of 5 ints {b_max, pair, wide, bn_cap, units_per_pair}; the first entry
  * (in b_max order) with b_max >= the batch size chooses the GEMM plan: pair = 1 CTA-pair kernels, 0 single-CTA
- * kernels; wide = 1 scan units of 512 limb columns, 0 never; bn_cap = largest limb-column tile (32..256);
- * units_per_pair = scan split target; -1 or 0 keeps the built-in choice.  Every plan computes identical results.
+ * kernels; wide = 1 scan units of 320 to 512 limb columns where a batch has more than 256, 0 never; bn_cap = largest
+ * limb-column tile (32..256); units_per_pair = scan split target; -1 or 0 keeps the built-in choice.  Every plan computes identical results.
  * alto_engine_new loads the committed table from $ALTO_TUNING or tuning.txt next to this library (lines
  * "rows_max b_max pair wide bn_cap units_per_pair", the rows of the smallest rows_max >= the engine's records).
  * n = 0 clears the table.  Returns 0, -1 for bad arguments, -4 on a device failure. */
