@@ -1,7 +1,8 @@
 #!/usr/bin/env python
 """Throughput of the AltoPIR answer path on B200: byte-exact QPS of answer batches.  The headline is 128-query
 batches on a 1 GiB database (32,768 records x 32 KB), the configuration of the reference's headline batch numbers;
-the same JSON line carries the 8 GiB (B = 1, 128, 1024) and 64 GiB (B = 128, 1024) databases under `configs`.
+the same JSON line carries the 8 GiB (B = 1 to 1024) and 64 GiB (B = 128, 1024) databases in brief under `configs`, and
+stderr all their fields.
 
 One step = one batch of --batch queries through the whole answer path (validate, limb split, scan, pack, tail).
 Every measurement times blocks of exactly --steps steps with CUDA events (a barrier and a synchronisation on both
@@ -586,6 +587,23 @@ def summarize(m, p, B, steps, world, dev, kern, e2e, plain, peaks, peak_src, tra
     }
 
 
+def brief(r):
+    """What the JSON line carries of a configuration beside the headline one (the rest goes to stderr): with all fields of
+    nine configurations the line had 28 KB, which readers that keep a bounded piece of the output do not find whole."""
+    return {
+        "config": {k: r["config"][k] for k in ("rows", "record_bytes", "batch")},
+        "value": r["value"], "ms_per_step": r["ms_per_step"], "steps": r["steps"], "blocks": r["blocks"],
+        "e2e": {k: r["e2e"][k] for k in ("value", "ms_per_step", "h2d_bytes_per_step", "d2h_bytes_per_step")},
+        "gpu_launches": r["gpu_launches"], "lanes": r["lanes"],
+        "roofline": {k: r["roofline"][k] for k in ("bound", "achieved", "unit", "frac")},
+        "kernels_ms": {k: r["kernels"][k]["avg_ms"] for k in ("gemms", "pack_gemm", "tail")},
+        "plain_per_query": {k: r["plain_per_query"][k] for k in ("qps", "p50_ms", "p99_ms", "batched_over_plain")},
+        "byte_exact": r["byte_exact"],
+        "clocks": {k: r["clocks"].get(k) for k in ("sm_mhz", "reasons")},
+        "vs_baseline": r["vs_baseline"],
+    }
+
+
 def lanes_for(lanes, rows, batch):
     """Batch lanes of the device-resident loop: two overlapping batches help while one record chunk of a batch's
     query limbs (4 bytes per record and frame, chunks of 32768 records) is a small part of the 126 MB L2; at 1024
@@ -730,7 +748,8 @@ def main_ours(a):
                           "lanes": lanes_for(lanes, rows, B),
                           "vs_baseline": r["value"] / pub[0] if pub else None,
                           "vs_baseline_ref": f"{pub[0]} QPS, {pub[1]}" if pub else None})
-                configs.append(r)
+                configs.append(brief(r))
+                print("detail " + json.dumps(r), file=sys.stderr)
                 print(f"config {rows} records, B = {B}: {r['value']:.0f} QPS device, {r['e2e']['value']:.0f} e2e, "
                       f"frac {r['roofline']['frac']:.3f}", file=sys.stderr, flush=True)
                 m.close()
